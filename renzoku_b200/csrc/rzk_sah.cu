@@ -10,177 +10,464 @@
 // bit for bit; a tree with less overlap than the Morton LBVH simply reaches the answer in
 // fewer steps.  Closest-hit queries keep the reference tree, whose visit order decides ties.
 //
-// Built on the host with binned SAH (32 bins on the centroid axis of largest extent; a
-// median split past depth 32 or when the centroids coincide), nodes numbered depth-first
-// with siblings adjacent, packed like the reference tree (two float4 per node slot).
+// Binned SAH: 32 bins on the centroid axis of largest extent; past depth 32 or when no split
+// separates the centroids, the median of the Morton order the slots came in.  Nodes are
+// numbered depth-first with siblings adjacent and packed like the reference tree (two float4
+// per node slot).
+//
+// Built on the device in two phases.  A node of more than kSmall triangles is split by one
+// block (bounds, bins in shared memory, stable partition), all such nodes of a level in one
+// launch; a node of at most kSmall triangles is finished by one warp, its boxes in shared
+// memory and its whole subtree built there without another launch.  Both phases stay short
+// because the top levels move the most data per block and there are few of them.  Every
+// result is independent of scheduling: bounds and bins are exact minima, maxima and counts,
+// the partition is stable, and a node's number follows from its range alone - an inner node
+// over the positions [begin, end) reached through `lefts` left turns has begin + lefts inner
+// nodes before it in depth-first order, so its children are nodes 1 + 2 (begin + lefts) and
+// the next.
 #include "rzk_internal.cuh"
 
 #include <algorithm>
 #include <cfloat>
-#include <cstring>
-#include <vector>
 
 namespace rzk {
 namespace {
 
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kBins = 32;          // one bin per lane of the warp that chooses the split
+constexpr int kMedianDepth = 32;   // deeper nodes are halved: depth stays under 32 + log2(n)
+constexpr int kSmall = 256;        // triangles whose subtree one warp builds
+constexpr int kLargeThreads = 1024;
+constexpr int kSmallWarps = 4;     // 4 x 10.8 KB of shared memory per block
+constexpr int kMaxLevels = 64;
+
+// A node to build: the triangles idx[begin, end), its node index, and depth | lefts << 8 |
+// buffer << 16 (which of the two index buffers holds the range).
+struct Task {
+    int begin, end, node, info;
+};
+static_assert(sizeof(Task) == 16, "one 16-byte load");
+
 struct Box {
-    float mn[3], mx[3];
-    void reset() {
-        for (int i = 0; i < 3; ++i) { mn[i] = FLT_MAX; mx[i] = -FLT_MAX; }
+    V3 mn, mx;
+    __device__ __forceinline__ void reset() {
+        mn = mk(FLT_MAX, FLT_MAX, FLT_MAX);
+        mx = mk(-FLT_MAX, -FLT_MAX, -FLT_MAX);
     }
-    void grow(const Box &b) {
-        for (int i = 0; i < 3; ++i) {
-            mn[i] = std::min(mn[i], b.mn[i]);
-            mx[i] = std::max(mx[i], b.mx[i]);
-        }
+    __device__ __forceinline__ void grow(V3 a, V3 b) {
+        mn = mk(fminf(mn.x, a.x), fminf(mn.y, a.y), fminf(mn.z, a.z));
+        mx = mk(fmaxf(mx.x, b.x), fmaxf(mx.y, b.y), fmaxf(mx.z, b.z));
     }
-    float area() const {
-        float dx = mx[0] - mn[0], dy = mx[1] - mn[1], dz = mx[2] - mn[2];
-        if (dx < 0.0f) return 0.0f;
-        return dx * dy + dy * dz + dz * dx;
+    __device__ __forceinline__ float area() const {
+        const float dx = mx.x - mn.x, dy = mx.y - mn.y, dz = mx.z - mn.z;
+        return dx < 0.0f ? 0.0f : dx * dy + dy * dz + dz * dx;
     }
 };
 
-struct Builder {
-    const std::vector<Box> &box;     // per sorted triangle slot
-    std::vector<float> cen;          // 3 per slot
-    std::vector<int> idx;            // slots, partitioned in place
-    std::vector<float4> out;         // 2 float4 per node slot; slot = node + 1
-    int next = 1;                    // next free node index (root = 0)
-    int max_depth = 0;
+__device__ __forceinline__ V3 centroid(float4 lo, float4 hi) {
+    return mk(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+}
+__device__ __forceinline__ V3 xyz(float4 f) { return mk(f.x, f.y, f.z); }
+__device__ __forceinline__ float comp(V3 v, int d) { return d == 0 ? v.x : d == 1 ? v.y : v.z; }
 
-    explicit Builder(const std::vector<Box> &b) : box(b) {}
+// floats as ints of the same order, for integer min / max reductions and atomics
+__device__ __forceinline__ int ord(float f) {
+    const int i = __float_as_int(f);
+    return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float unord(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
 
-    static float bits(int a) {
-        float f;
-        std::memcpy(&f, &a, sizeof(f));
-        return f;
+__device__ __forceinline__ V3 warp_min(V3 v) {
+    return mk(unord(__reduce_min_sync(kFull, ord(v.x))), unord(__reduce_min_sync(kFull, ord(v.y))),
+              unord(__reduce_min_sync(kFull, ord(v.z))));
+}
+__device__ __forceinline__ V3 warp_max(V3 v) {
+    return mk(unord(__reduce_max_sync(kFull, ord(v.x))), unord(__reduce_max_sync(kFull, ord(v.y))),
+              unord(__reduce_max_sync(kFull, ord(v.z))));
+}
+
+// The axis of largest centroid extent and the binning along it.
+struct Binning {
+    int axis;
+    float lo, k, ext;
+    __device__ __forceinline__ void set(const Box &c) {
+        const V3 e = sub(c.mx, c.mn);
+        axis = 0;
+        if (e.y > e.x) axis = 1;
+        if (e.z > comp(e, axis)) axis = 2;
+        ext = comp(e, axis);
+        lo = comp(c.mn, axis);
+        k = kBins / ext;
     }
-    void write(int node, const Box &b, int a) {
-        out[2 * (node + 1)] = make_float4(b.mn[0], b.mn[1], b.mn[2], bits(a));
-        out[2 * (node + 1) + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], bits(0));
-    }
-
-    // returns the node's box; the node's record is written here
-    Box build(int node, int begin, int end, int depth) {
-        max_depth = std::max(max_depth, depth);
-        Box nb;
-        nb.reset();
-        for (int i = begin; i < end; ++i) nb.grow(box[idx[i]]);
-        if (end - begin == 1) {
-            write(node, nb, -1 - idx[begin]);
-            return nb;
-        }
-        float cmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (int i = begin; i < end; ++i)
-            for (int d = 0; d < 3; ++d) {
-                cmn[d] = std::min(cmn[d], cen[3 * idx[i] + d]);
-                cmx[d] = std::max(cmx[d], cen[3 * idx[i] + d]);
-            }
-        int axis = 0;
-        for (int d = 1; d < 3; ++d)
-            if (cmx[d] - cmn[d] > cmx[axis] - cmn[axis]) axis = d;
-        int mid = -1;
-        const float ext = cmx[axis] - cmn[axis];
-        if (ext > 0.0f && depth < 32) {
-            constexpr int B = 32;
-            Box bb[B];
-            int cnt[B] = {0};
-            for (int b = 0; b < B; ++b) bb[b].reset();
-            const float k = B / ext;
-            auto bin_of = [&](int s) {
-                int b = (int)((cen[3 * s + axis] - cmn[axis]) * k);
-                return std::min(std::max(b, 0), B - 1);
-            };
-            for (int i = begin; i < end; ++i) {
-                const int b = bin_of(idx[i]);
-                cnt[b]++;
-                bb[b].grow(box[idx[i]]);
-            }
-            float right_area[B];
-            int right_cnt[B];
-            Box acc;
-            acc.reset();
-            int c = 0;
-            for (int b = B - 1; b > 0; --b) {
-                acc.grow(bb[b]);
-                c += cnt[b];
-                right_area[b] = acc.area();
-                right_cnt[b] = c;
-            }
-            acc.reset();
-            c = 0;
-            float best = FLT_MAX;
-            int best_b = -1;
-            for (int b = 0; b < B - 1; ++b) {
-                acc.grow(bb[b]);
-                c += cnt[b];
-                if (c == 0 || right_cnt[b + 1] == 0) continue;
-                const float cost = c * acc.area() + right_cnt[b + 1] * right_area[b + 1];
-                if (cost < best) { best = cost; best_b = b; }
-            }
-            if (best_b >= 0) {
-                int *first = idx.data() + begin, *last = idx.data() + end;
-                int *m = std::partition(first, last, [&](int s) { return bin_of(s) <= best_b; });
-                mid = (int)(m - idx.data());
-                if (mid == begin || mid == end) mid = -1;
-            }
-        }
-        if (mid < 0) {   // coincident centroids or too deep: median by centroid
-            mid = (begin + end) / 2;
-            std::nth_element(idx.begin() + begin, idx.begin() + mid, idx.begin() + end,
-                             [&](int x, int y) { return cen[3 * x + axis] < cen[3 * y + axis]; });
-        }
-        const int left = next;
-        next += 2;
-        build(left, begin, mid, depth + 1);
-        build(left + 1, mid, end, depth + 1);
-        write(node, nb, left);
-        return nb;
+    __device__ __forceinline__ int bin(V3 cen) const {
+        const int b = (int)((comp(cen, axis) - lo) * k);
+        return min(max(b, 0), kBins - 1);
     }
 };
+
+// Lane b holds bin b's box and count.  Returns the bin after which to split (the first of
+// least cost), or -1 if none separates the triangles; `left` = the triangles up to it.
+__device__ __forceinline__ int choose_split(const Box &bin, int count, int lane, int &left) {
+    Box l = bin, r = bin;
+    int lc = count, rc = count;
+#pragma unroll
+    for (int o = 1; o < kBins; o <<= 1) {
+        const V3 a = mk(__shfl_up_sync(kFull, l.mn.x, o), __shfl_up_sync(kFull, l.mn.y, o), __shfl_up_sync(kFull, l.mn.z, o));
+        const V3 b = mk(__shfl_up_sync(kFull, l.mx.x, o), __shfl_up_sync(kFull, l.mx.y, o), __shfl_up_sync(kFull, l.mx.z, o));
+        const V3 c = mk(__shfl_down_sync(kFull, r.mn.x, o), __shfl_down_sync(kFull, r.mn.y, o), __shfl_down_sync(kFull, r.mn.z, o));
+        const V3 d = mk(__shfl_down_sync(kFull, r.mx.x, o), __shfl_down_sync(kFull, r.mx.y, o), __shfl_down_sync(kFull, r.mx.z, o));
+        const int n = __shfl_up_sync(kFull, lc, o), m = __shfl_down_sync(kFull, rc, o);
+        if (lane >= o) { l.grow(a, b); lc += n; }
+        if (lane + o < kBins) { r.grow(c, d); rc += m; }
+    }
+    const float ra = __shfl_down_sync(kFull, r.area(), 1);
+    const int rn = __shfl_down_sync(kFull, rc, 1);
+    float cost = FLT_MAX;
+    if (lane < kBins - 1 && lc > 0 && rn > 0) cost = lc * l.area() + rn * ra;
+    const int best = __reduce_min_sync(kFull, ord(cost));
+    if (!(unord(best) < FLT_MAX)) return -1;
+    const int b = __ffs(__ballot_sync(kFull, ord(cost) == best)) - 1;
+    left = __shfl_sync(kFull, lc, b);
+    return b;
+}
+
+__device__ __forceinline__ void write_node(float4 *out, int node, const Box &b, int code) {
+    out[2 * (node + 1)] = make_float4(b.mn.x, b.mn.y, b.mn.z, __int_as_float(code));
+    out[2 * (node + 1) + 1] = make_float4(b.mx.x, b.mx.y, b.mx.z, __int_as_float(0));
+}
+
+// Box of every sorted triangle slot as two float4 (one 32-byte sector), and the initial
+// order: the slots' own, which is the Morton order.
+__global__ void sah_boxes_kernel(int n, const int *perm, const float *bmin, const float *bmax, float4 *box, int *idx) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const size_t t = perm[s];
+    box[2 * (size_t)s] = make_float4(bmin[3 * t], bmin[3 * t + 1], bmin[3 * t + 2], 0.0f);
+    box[2 * (size_t)s + 1] = make_float4(bmax[3 * t], bmax[3 * t + 1], bmax[3 * t + 2], 0.0f);
+    idx[s] = s;
+}
+
+__global__ void sah_root_kernel(int n, Task *large, int *n_large, Task *small, int *n_small) {
+    const Task t{0, n, 0, 0};
+    if (n > kSmall) { large[0] = t; *n_large = 1; } else { small[0] = t; *n_small = 1; }
+}
+
+// One block per node of more than kSmall triangles: its node record, its triangles
+// partitioned into the other index buffer, and its children appended to the next level's
+// list or to the small list.
+__global__ void __launch_bounds__(kLargeThreads) sah_large_kernel(const float4 *box, int *idx0, int *idx1,
+                                                                  const Task *tasks, const int *n_tasks, Task *next,
+                                                                  int *n_next, Task *small, int *n_small, float4 *out) {
+    constexpr int W = kLargeThreads / 32;
+    __shared__ int red[W][12];
+    __shared__ int bins[kBins][7];
+    __shared__ int wcnt[W];
+    __shared__ Binning s_bin;
+    __shared__ int s_best, s_left;
+    __shared__ Box s_box;
+    if ((int)blockIdx.x >= *n_tasks) return;
+    const Task t = tasks[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int depth = t.info & 255, lefts = (t.info >> 8) & 255, buf = t.info >> 16;
+    const int *in = buf ? idx1 : idx0;
+    int *to = buf ? idx0 : idx1;
+
+    Box b, c;
+    b.reset();
+    c.reset();
+    for (int i = t.begin + tid; i < t.end; i += kLargeThreads) {
+        const size_t s = in[i];
+        const float4 lo = box[2 * s], hi = box[2 * s + 1];
+        const V3 m = centroid(lo, hi);
+        b.grow(xyz(lo), xyz(hi));
+        c.grow(m, m);
+    }
+    b.mn = warp_min(b.mn);
+    b.mx = warp_max(b.mx);
+    c.mn = warp_min(c.mn);
+    c.mx = warp_max(c.mx);
+    if (lane == 0) {
+        const V3 v[4] = {b.mn, b.mx, c.mn, c.mx};
+        for (int k = 0; k < 4; ++k) {
+            red[w][3 * k] = ord(v[k].x);
+            red[w][3 * k + 1] = ord(v[k].y);
+            red[w][3 * k + 2] = ord(v[k].z);
+        }
+    }
+    if (tid < kBins * 7) {
+        const int f = tid % 7;
+        bins[tid / 7][f] = f < 3 ? ord(FLT_MAX) : f < 6 ? ord(-FLT_MAX) : 0;
+    }
+    __syncthreads();
+    if (w == 0) {   // lane = warp of the block
+        auto get = [&](int k) { return mk(unord(red[lane][k]), unord(red[lane][k + 1]), unord(red[lane][k + 2])); };
+        b.mn = warp_min(get(0));
+        b.mx = warp_max(get(3));
+        c.mn = warp_min(get(6));
+        c.mx = warp_max(get(9));
+        if (lane == 0) {
+            s_box = b;
+            s_bin.set(c);
+            s_best = -1;
+            s_left = (t.end - t.begin) / 2;
+        }
+    }
+    __syncthreads();
+    const Binning bn = s_bin;
+    if (bn.ext > 0.0f && depth < kMedianDepth) {
+        // consecutive positions are close along the Morton curve and fall into few bins: the
+        // warp reduces bin by bin and one lane updates the block's bin
+        for (int i0 = t.begin + 32 * w; i0 < t.end; i0 += kLargeThreads) {
+            const int i = i0 + lane;
+            int bin = -1;
+            float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+            if (i < t.end) {
+                const size_t s = in[i];
+                lo = box[2 * s];
+                hi = box[2 * s + 1];
+                bin = bn.bin(centroid(lo, hi));
+            }
+            unsigned todo = __ballot_sync(kFull, bin >= 0);
+            while (todo) {
+                const int cur = __shfl_sync(kFull, bin, __ffs(todo) - 1);
+                const bool mine = bin == cur;
+                const unsigned group = __ballot_sync(kFull, mine);
+                const int a0 = __reduce_min_sync(kFull, mine ? ord(lo.x) : INT_MAX);
+                const int a1 = __reduce_min_sync(kFull, mine ? ord(lo.y) : INT_MAX);
+                const int a2 = __reduce_min_sync(kFull, mine ? ord(lo.z) : INT_MAX);
+                const int a3 = __reduce_max_sync(kFull, mine ? ord(hi.x) : INT_MIN);
+                const int a4 = __reduce_max_sync(kFull, mine ? ord(hi.y) : INT_MIN);
+                const int a5 = __reduce_max_sync(kFull, mine ? ord(hi.z) : INT_MIN);
+                if (lane < 7) {
+                    int *p = &bins[cur][lane];
+                    const int v = lane == 0 ? a0 : lane == 1 ? a1 : lane == 2 ? a2 : lane == 3 ? a3 : lane == 4 ? a4 : a5;
+                    if (lane < 3) atomicMin(p, v);
+                    else if (lane < 6) atomicMax(p, v);
+                    else atomicAdd(p, __popc(group));
+                }
+                todo &= ~group;
+            }
+        }
+        __syncthreads();
+        if (w == 0) {
+            Box bb;
+            bb.mn = mk(unord(bins[lane][0]), unord(bins[lane][1]), unord(bins[lane][2]));
+            bb.mx = mk(unord(bins[lane][3]), unord(bins[lane][4]), unord(bins[lane][5]));
+            int left = 0;
+            const int best = choose_split(bb, bins[lane][6], lane, left);
+            if (lane == 0 && best >= 0) { s_best = best; s_left = left; }
+        }
+        __syncthreads();
+    }
+    const int best = s_best, mid = t.begin + s_left;
+    int lrun = t.begin, rrun = mid;   // next free left and right position
+    for (int i0 = t.begin; i0 < t.end; i0 += kLargeThreads) {
+        const int i = i0 + tid;
+        int s = 0;
+        bool left = false;
+        if (i < t.end) {
+            s = in[i];
+            left = best >= 0 ? bn.bin(centroid(box[2 * (size_t)s], box[2 * (size_t)s + 1])) <= best : i < mid;
+        }
+        const unsigned m = __ballot_sync(kFull, left);
+        if (lane == 0) wcnt[w] = __popc(m);
+        __syncthreads();
+        const int mine = wcnt[lane];
+        const int before = __reduce_add_sync(kFull, lane < w ? mine : 0);
+        const int total = __reduce_add_sync(kFull, mine);
+        const int lrank = before + __popc(m & ((1u << lane) - 1u));
+        if (i < t.end) to[left ? lrun + lrank : rrun + (tid - lrank)] = s;
+        lrun += total;
+        rrun += min(kLargeThreads, t.end - i0) - total;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        const int child = 1 + 2 * (t.begin + lefts);
+        write_node(out, t.node, s_box, child);
+        for (int k = 0; k < 2; ++k) {
+            Task n;
+            n.begin = k ? mid : t.begin;
+            n.end = k ? t.end : mid;
+            n.node = child + k;
+            n.info = (depth + 1) | (lefts + (k ? 0 : 1)) << 8 | (buf ^ 1) << 16;
+            if (n.end - n.begin > kSmall) next[atomicAdd(n_next, 1)] = n;
+            else small[atomicAdd(n_small, 1)] = n;
+        }
+    }
+}
+
+// One warp per subtree of at most kSmall triangles.
+struct SmallMem {
+    float4 box[2 * kSmall];
+    int slot[kSmall];
+    uint8_t order[2][kSmall];   // local triangles in position order, and the partition's target
+    Task stack[64];             // pending right children, positions relative to the subtree's
+};
+
+__global__ void __launch_bounds__(32 * kSmallWarps) sah_small_kernel(const float4 *box, const int *idx0, const int *idx1,
+                                                                     const Task *tasks, const int *n_tasks, float4 *out,
+                                                                     int *max_depth) {
+    __shared__ SmallMem mem[kSmallWarps];
+    static_assert(kSmall <= 256, "order holds bytes");
+    const int lane = threadIdx.x & 31;
+    SmallMem &m = mem[threadIdx.x >> 5];
+    const int total = *n_tasks, step = gridDim.x * kSmallWarps;
+    for (int k = blockIdx.x * kSmallWarps + (threadIdx.x >> 5); k < total; k += step) {
+        const Task t = tasks[k];
+        const int *in = t.info >> 16 ? idx1 : idx0;
+        const int n = t.end - t.begin;
+        for (int i = lane; i < n; i += 32) {
+            const int s = in[t.begin + i];
+            m.slot[i] = s;
+            m.box[2 * i] = box[2 * (size_t)s];
+            m.box[2 * i + 1] = box[2 * (size_t)s + 1];
+            m.order[0][i] = (uint8_t)i;
+        }
+        __syncwarp();
+        int begin = 0, end = n, node = t.node, depth = t.info & 255, lefts = (t.info >> 8) & 255, top = 0;
+        int deepest = depth;
+        for (;;) {
+            const int cnt = end - begin;
+            Box b, c;
+            b.reset();
+            c.reset();
+            for (int i = begin + lane; i < end; i += 32) {
+                const int q = m.order[0][i];
+                const float4 lo = m.box[2 * q], hi = m.box[2 * q + 1];
+                const V3 ce = centroid(lo, hi);
+                b.grow(xyz(lo), xyz(hi));
+                c.grow(ce, ce);
+            }
+            b.mn = warp_min(b.mn);
+            b.mx = warp_max(b.mx);
+            if (cnt == 1) {
+                deepest = max(deepest, depth);
+                if (lane == 0) write_node(out, node, b, -1 - m.slot[m.order[0][begin]]);
+                if (top == 0) break;
+                const Task e = m.stack[--top];
+                __syncwarp();
+                begin = e.begin;
+                end = e.end;
+                node = e.node;
+                depth = e.info & 255;
+                lefts = e.info >> 8;
+                continue;
+            }
+            c.mn = warp_min(c.mn);
+            c.mx = warp_max(c.mx);
+            Binning bn;
+            bn.set(c);
+            int best = -1, left = cnt / 2;
+            if (bn.ext > 0.0f && depth < kMedianDepth) {
+                Box bb;   // this lane's bin
+                bb.reset();
+                int bc = 0;
+                for (int i = begin; i < end; ++i) {
+                    const int q = m.order[0][i];
+                    const float4 lo = m.box[2 * q], hi = m.box[2 * q + 1];
+                    if (bn.bin(centroid(lo, hi)) == lane) {
+                        bb.grow(xyz(lo), xyz(hi));
+                        ++bc;
+                    }
+                }
+                int nl = 0;
+                best = choose_split(bb, bc, lane, nl);
+                if (best >= 0) left = nl;
+            }
+            if (best >= 0) {   // stable partition (a median split keeps the order)
+                int lrun = begin, rrun = begin + left;
+                for (int i0 = begin; i0 < end; i0 += 32) {
+                    const int i = i0 + lane;
+                    int q = 0;
+                    bool l = false;
+                    if (i < end) {
+                        q = m.order[0][i];
+                        l = bn.bin(centroid(m.box[2 * q], m.box[2 * q + 1])) <= best;
+                    }
+                    const unsigned lm = __ballot_sync(kFull, l);
+                    const int lrank = __popc(lm & ((1u << lane) - 1u));
+                    if (i < end) m.order[1][l ? lrun + lrank : rrun + (lane - lrank)] = (uint8_t)q;
+                    lrun += __popc(lm);
+                    rrun += min(32, end - i0) - __popc(lm);
+                }
+                __syncwarp();
+                for (int i = begin + lane; i < end; i += 32) m.order[0][i] = m.order[1][i];
+                __syncwarp();
+            }
+            const int child = 1 + 2 * (t.begin + begin + lefts);
+            if (lane == 0) {
+                write_node(out, node, b, child);
+                m.stack[top] = Task{begin + left, end, child + 1, (depth + 1) | lefts << 8};
+            }
+            __syncwarp();
+            ++top;
+            end = begin + left;
+            node = child;
+            ++depth;
+            ++lefts;
+        }
+        if (lane == 0) atomicMax(max_depth, deepest);
+        __syncwarp();
+    }
+}
 
 }  // namespace
 
 rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st) {
     const int n = s->n_tris;
     if (n <= 0) return RZK_OK;
-    std::vector<float> bmin(3 * (size_t)n), bmax(3 * (size_t)n);
-    std::vector<int> perm(n);
-    RZK_CUDA_TRY(cudaMemcpyAsync(bmin.data(), s->d_bmin, sizeof(float) * bmin.size(), cudaMemcpyDeviceToHost, st));
-    RZK_CUDA_TRY(cudaMemcpyAsync(bmax.data(), s->d_bmax, sizeof(float) * bmax.size(), cudaMemcpyDeviceToHost, st));
-    RZK_CUDA_TRY(cudaMemcpyAsync(perm.data(), s->d_perm, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-    RZK_CUDA_TRY(cudaStreamSynchronize(st));
-    std::vector<Box> box(n);
-    for (int slot = 0; slot < n; ++slot) {
-        const int t = perm[slot];
-        for (int d = 0; d < 3; ++d) {
-            box[slot].mn[d] = bmin[3 * (size_t)t + d];
-            box[slot].mx[d] = bmax[3 * (size_t)t + d];
-        }
-    }
-    Builder b(box);
-    b.cen.resize(3 * (size_t)n);
-    for (int slot = 0; slot < n; ++slot)
-        for (int d = 0; d < 3; ++d) b.cen[3 * (size_t)slot + d] = 0.5f * (box[slot].mn[d] + box[slot].mx[d]);
-    b.idx.resize(n);
-    for (int i = 0; i < n; ++i) b.idx[i] = i;
-    const int n_nodes = 2 * n - 1;
-    b.out.assign(2 * ((size_t)n_nodes + 1), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    b.build(0, 0, n, 0);
-    if (b.max_depth >= STACK_CAP - 2) return RZK_ERR_STACK;
-    if (s->d_trav) {
+    const size_t bytes = sizeof(float4) * 4 * (size_t)n;   // 2n - 1 nodes and the unused slot 0
+    if (s->d_trav && s->trav_bytes != bytes) {
         cudaFree(s->d_trav);
+        s->d_trav = nullptr;
         s->device_bytes -= s->trav_bytes;
     }
-    s->d_trav = nullptr;
-    s->trav_bytes = sizeof(float4) * b.out.size();
-    RZK_CUDA_TRY(cudaMalloc((void **)&s->d_trav, s->trav_bytes));
-    RZK_CUDA_TRY(cudaMemcpyAsync(s->d_trav, b.out.data(), sizeof(float4) * b.out.size(), cudaMemcpyHostToDevice, st));
+    if (!s->d_trav) {
+        s->trav_bytes = 0;
+        RZK_CUDA_TRY(cudaMalloc((void **)&s->d_trav, bytes));
+        s->trav_bytes = bytes;
+        s->device_bytes += bytes;
+    }
+    // nodes of one level are disjoint ranges of more than kSmall triangles; every small node
+    // holds at least one triangle of its own
+    const int max_large = n / (kSmall + 1) + 1;
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t o_idx0 = up(2 * sizeof(float4) * (size_t)n), o_idx1 = o_idx0 + up(sizeof(int) * (size_t)n);
+    const size_t o_small = o_idx1 + up(sizeof(int) * (size_t)n), o_l0 = o_small + up(sizeof(Task) * (size_t)n);
+    const size_t o_l1 = o_l0 + up(sizeof(Task) * (size_t)max_large), o_cnt = o_l1 + up(sizeof(Task) * (size_t)max_large);
+    char *buf = nullptr;
+    RZK_CUDA_TRY(cudaMalloc((void **)&buf, o_cnt + sizeof(int) * (kMaxLevels + 3)));
+    struct Free { char *p; ~Free() { cudaFree(p); } } guard{buf};
+    float4 *box = (float4 *)buf;
+    int *idx0 = (int *)(buf + o_idx0), *idx1 = (int *)(buf + o_idx1);
+    Task *small = (Task *)(buf + o_small), *large[2] = {(Task *)(buf + o_l0), (Task *)(buf + o_l1)};
+    int *n_small = (int *)(buf + o_cnt), *max_depth = n_small + 1,
+        *n_large = n_small + 2;   // n_large[level]
+    RZK_CUDA_TRY(cudaMemsetAsync(n_small, 0, sizeof(int) * (kMaxLevels + 3), st));
+    RZK_CUDA_TRY(cudaMemsetAsync(s->d_trav, 0, 2 * sizeof(float4), st));
+    sah_boxes_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, s->d_perm, s->d_bmin, s->d_bmax, box, idx0);
+    sah_root_kernel<<<1, 1, 0, st>>>(n, large[0], n_large, small, n_small);
+    RZK_CUDA_TRY(cudaGetLastError());
+    int pending = n > kSmall ? 1 : 0;
+    for (int level = 0; pending && level < kMaxLevels; ++level) {
+        const int grid = level < 30 ? std::min(max_large, 1 << level) : max_large;
+        sah_large_kernel<<<grid, kLargeThreads, 0, st>>>(box, idx0, idx1, large[level & 1], n_large + level,
+                                                         large[(level + 1) & 1], n_large + level + 1, small, n_small,
+                                                         s->d_trav);
+        RZK_CUDA_TRY(cudaGetLastError());
+        // a level has nodes only if the one before it had: look once in four levels, the first
+        // time when an even split would be done
+        if ((level & 3) == 3 && (kSmall << level) >= n) {
+            RZK_CUDA_TRY(cudaMemcpyAsync(&pending, n_large + level + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+            RZK_CUDA_TRY(cudaStreamSynchronize(st));
+        }
+    }
+    sah_small_kernel<<<(n + 128 * kSmallWarps - 1) / (128 * kSmallWarps), 32 * kSmallWarps, 0, st>>>(
+        box, idx0, idx1, small, n_small, s->d_trav, max_depth);
+    RZK_CUDA_TRY(cudaGetLastError());
+    RZK_CUDA_TRY(cudaMemcpyAsync(&s->trav_depth, max_depth, sizeof(int), cudaMemcpyDeviceToHost, st));
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
-    s->trav_depth = b.max_depth;
-    s->device_bytes += s->trav_bytes;
-    return RZK_OK;
+    return s->trav_depth >= STACK_CAP - 2 ? RZK_ERR_STACK : RZK_OK;
 }
 
 }  // namespace rzk
