@@ -82,30 +82,34 @@ __device__ Rgb first_bounce(const DevScene &s, const GuideRecv &r, const rzk_mat
     float pdf;
     light_sample_point(L, g, q, qn, pdf);
     if (pdf > 0.0f) {
-        Ray sr = make_ray(p, sub(q, p));
-        const float tmax = len(sub(q, p)) - s.tmin;
-        if (!any_hit<STRIDE, false, true>(s, sr, s.tmin, tmax, stk)) {
-            const V3 wi = unit(sub(q, p));
-            const Rgb Le = light_query(L, q, qn, neg(wi));
-            const float G = form_factor_abs(p, pn, q, qn);
-            if (G > 0.0f) {
-                const Rgb brdf = brdf_eval(m, r.uvn, r.wo, wi);
-                const float dsp = brdf_pdf(m, r.uvn, r.wo, wi, rho_d, rho_s);
-                const V3 pq = sub(q, p);
-                const float sq = pq.x * pq.x + pq.y * pq.y + pq.z * pq.z;
-                const float w1 = balance(pdf * sq / fabsf(dot(unit(sub(p, q)), qn)), dsp);
-                Lo = cadd(Lo, cmul(cscl(Le, w1 * G / pdf), brdf));
+        // the term is formed first: where it is exactly zero (the light seen from behind, or
+        // below the receiver's horizon) it adds nothing whatever the visibility
+        const V3 wi = unit(sub(q, p));
+        const Rgb Le = light_query(L, q, qn, neg(wi));
+        const float G = form_factor_abs(p, pn, q, qn);
+        if (G > 0.0f) {
+            const Rgb brdf = brdf_eval(m, r.uvn, r.wo, wi);
+            const float dsp = brdf_pdf(m, r.uvn, r.wo, wi, rho_d, rho_s);
+            const V3 pq = sub(q, p);
+            const float sq = pq.x * pq.x + pq.y * pq.y + pq.z * pq.z;
+            const float w1 = balance(pdf * sq / fabsf(dot(unit(sub(p, q)), qn)), dsp);
+            const Rgb term = cmul(cscl(Le, w1 * G / pdf), brdf);
+            if (!cblack(term)) {
+                Ray sr = make_ray(p, sub(q, p));
+                const float tmax = len(sub(q, p)) - s.tmin;
+                if (!any_hit<STRIDE, false, true>(s, sr, s.tmin, tmax, stk)) Lo = cadd(Lo, term);
             }
         }
     }
-    // a direction from the BRDF that reaches this light
+    // a direction from the BRDF that reaches this light: the closest hit is on the light only
+    // if the ray hits one of the light's own triangles, which few do
     V3 wi;
     float dsp;
     (void)brdf_sample(m, r.uvn, r.wo, g, wi, dsp);
     if (dsp > 0.0f) {
         Ray ray = make_ray(p, wi);
         HitGeo h;
-        if (trace_closest(s, ray, stk, h) && h.light == k) {
+        if (light_hit(L, ray, s.tmin) && trace_closest(s, ray, stk, h) && h.light == k) {
             const V3 q2 = add(p, scl(wi, h.t));
             const V3 qn2 = h.ns;
             const Rgb Le = light_query(L, q2, qn2, neg(wi));

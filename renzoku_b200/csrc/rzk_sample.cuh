@@ -144,6 +144,21 @@ __device__ __forceinline__ Rgb light_query(const DevLight &L, V3 p, V3 n, V3 wo)
     return crgb(L.emit.x, L.emit.y, L.emit.z);
 }
 
+// Whether a ray's triangle test passes on one of the light's triangles (the record the scene's
+// traversal reads, rebuilt with the same operations).  False means that no hit of the ray can
+// be on this light; true says nothing about what lies in front of it.
+__device__ __forceinline__ bool light_hit(const DevLight &L, const Ray &r, float tmin) {
+    for (int k = 0; k < L.n_tris; ++k) {
+        const float4 p0 = L.p0[k], p1 = L.p1[k], p2 = L.p2[k];
+        const V3 o = mk(p0.x, p0.y, p0.z);
+        const V3 a = sub(o, mk(p1.x, p1.y, p1.z)), b = sub(o, mk(p2.x, p2.y, p2.z));
+        if (tri_hit<false>(make_float4(p0.x, p0.y, p0.z, a.x), make_float4(a.y, a.z, b.x, b.y),
+                           make_float4(b.z, 0.0f, 0.0f, 0.0f), r, tmin, RAY_TMAX, nullptr, nullptr, nullptr))
+            return true;
+    }
+    return false;
+}
+
 // Surface::sample -> Quad::sample (quad.cc:75-87) / Triangle::sample (triangle.cc:298-308),
 // the normal flipped on a flipped surface (surface.cc:98-102)
 __device__ __forceinline__ void light_sample_point(const DevLight &L, Rng &g, V3 &q, V3 &qn, float &pdf) {
