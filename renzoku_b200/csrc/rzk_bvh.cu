@@ -456,9 +456,9 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
     size_t o_box = carve(sizeof(float) * 6 * 1024 + 64);
     size_t o_total = carve(64);
     size_t o_scan = carve(scan_bytes);
-    char *scratch = nullptr;
-    RZK_CUDA_TRY(cudaMalloc((void **)&scratch, scratch_bytes));
-    struct Free { char *p; ~Free() { if (p) cudaFree(p); } } guard{scratch};
+    CallScratch mem;
+    RZK_CUDA_TRY(mem.alloc(scratch_bytes, st));
+    char *scratch = mem.get();
     uint32_t *keys2 = (uint32_t *)(scratch + o_keys2);
     int *vals2 = (int *)(scratch + o_vals2);
     int *hist = (int *)(scratch + o_hist);

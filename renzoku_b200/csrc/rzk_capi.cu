@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -15,6 +16,62 @@ static thread_local char g_last_error[512] = "";
 void set_last_cuda_error(cudaError_t e, const char *what, const char *file, int line) {
     snprintf(g_last_error, sizeof(g_last_error), "%s: %s (%s:%d)", cudaGetErrorString(e), what,
              file, line);
+}
+
+namespace {
+
+constexpr int kPoolDevices = 64;
+struct DevicePool {
+    std::mutex lock;
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+};
+DevicePool g_pools[kPoolDevices];
+
+}  // namespace
+
+cudaError_t CallScratch::alloc(size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kPoolDevices) return cudaErrorInvalidDevice;
+    DevicePool &d = g_pools[dev];
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> g(d.lock);
+        if (!d.pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t p = nullptr;
+            if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
+            unsigned long long keep = kPoolKeep;
+            if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+                cudaMemPoolDestroy(p);
+                return e;
+            }
+            d.pool = p;
+        }
+        pool = d.pool;
+    }
+    e = cudaMallocFromPoolAsync(&p_, bytes > 0 ? bytes : 1, pool, st);
+    if (e != cudaSuccess) p_ = nullptr;
+    st_ = st;
+    return e;
+}
+
+void pool_context_created(int device) {
+    if (device < 0 || device >= kPoolDevices) return;
+    std::lock_guard<std::mutex> g(g_pools[device].lock);
+    g_pools[device].contexts++;
+}
+
+void pool_context_destroyed(int device) {
+    if (device < 0 || device >= kPoolDevices) return;
+    DevicePool &d = g_pools[device];
+    std::lock_guard<std::mutex> g(d.lock);
+    if (--d.contexts == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
 }
 
 rzk_status launch_occluded(const DevScene &s, const float *p, const float *q, int n, uint8_t *out,
@@ -80,6 +137,7 @@ rzk_status rzk_context_create(int device, rzk_context **out) {
         delete c;
         return RZK_ERR_CUDA;
     }
+    pool_context_created(device);
     *out = c;
     return RZK_OK;
 }
@@ -92,6 +150,7 @@ rzk_status rzk_context_destroy(rzk_context *c) {
     if (c->d_stage) cudaFree(c->d_stage);
     if (c->d_work) cudaFree(c->d_work);
     if (c->d_order) cudaFree(c->d_order);
+    pool_context_destroyed(c->device);
     delete c;
     return RZK_OK;
 }

@@ -311,9 +311,13 @@ __global__ void argmin_kernel(const float *D, int cols, int count, int *owner) {
 
 template <class T>
 struct DevBuf {
+    CallScratch mem;
     T *p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
-    cudaError_t alloc(size_t n) { return cudaMalloc((void **)&p, sizeof(T) * (n > 0 ? n : 1)); }
+    cudaError_t alloc(size_t n, cudaStream_t st) {
+        const cudaError_t e = mem.alloc(sizeof(T) * n, st);
+        p = (T *)mem.get();
+        return e;
+    }
 };
 
 }  // namespace
@@ -324,7 +328,7 @@ static rzk_status column_stats_and_alphas(const float *mat, int rows, int cols, 
     if (cols <= 0) return RZK_OK;
     if (rows <= 0) return RZK_ERR_INVALID;
     DevBuf<float> buf;   // [rmag: cols | u: rows | c]
-    RZK_CUDA_TRY(buf.alloc((size_t)cols + rows + 1));
+    RZK_CUDA_TRY(buf.alloc((size_t)cols + rows + 1, st));
     float *rmag = buf.p, *u = rmag + cols, *c0 = u + rows;
     const int grid = (cols + kColTile - 1) / kColTile;
     column_kernel<false><<<grid, kStatThreads, 0, st>>>(mat, rows, cols, rmag, col_norms, flat_norms, nullptr, nullptr,
@@ -358,8 +362,8 @@ rzk_status cluster_by_sampling(const float *mat, int rows, int cols, int num_clu
         return RZK_OK;
     }
     DevBuf<float> alphas, nm;
-    RZK_CUDA_TRY(alphas.alloc(cols));
-    RZK_CUDA_TRY(nm.alloc(cols));
+    RZK_CUDA_TRY(alphas.alloc(cols, st));
+    RZK_CUDA_TRY(nm.alloc(cols, st));
     rzk_status e = column_stats_and_alphas(mat, rows, cols, alphas.p, nullptr, nm.p, st);
     if (e != RZK_OK) return e;
     std::vector<float> a(cols);
@@ -401,12 +405,12 @@ rzk_status cluster_by_sampling(const float *mat, int rows, int cols, int num_clu
     const size_t n3 = 3 * (size_t)rows;
     DevBuf<int> d_cen, d_owner;
     DevBuf<float> d_w, K, kn, D;
-    RZK_CUDA_TRY(d_cen.alloc(count));
-    RZK_CUDA_TRY(d_w.alloc(count));
-    RZK_CUDA_TRY(K.alloc(n3 * count));
-    RZK_CUDA_TRY(kn.alloc(count));
-    RZK_CUDA_TRY(d_owner.alloc(cols));
-    RZK_CUDA_TRY(D.alloc((size_t)cols * count));
+    RZK_CUDA_TRY(d_cen.alloc(count, st));
+    RZK_CUDA_TRY(d_w.alloc(count, st));
+    RZK_CUDA_TRY(K.alloc(n3 * count, st));
+    RZK_CUDA_TRY(kn.alloc(count, st));
+    RZK_CUDA_TRY(d_owner.alloc(cols, st));
+    RZK_CUDA_TRY(D.alloc((size_t)cols * count, st));
     RZK_CUDA_TRY(cudaMemcpyAsync(d_cen.p, cen.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
     RZK_CUDA_TRY(cudaMemcpyAsync(d_w.p, w.data(), sizeof(float) * count, cudaMemcpyHostToDevice, st));
     size_t tot = n3 * count;

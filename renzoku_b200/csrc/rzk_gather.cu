@@ -909,13 +909,13 @@ rzk_status launch_mean(rzk_context *ctx, const DevScene &s, const rzk_receiver *
                        cudaStream_t st) {
     if (n_pairs <= 0 || n_recv <= 0 || n_vpl <= 0) { *h_mean = 0.0; return RZK_OK; }
     int nb = (n_pairs + kMeanBlock - 1) / kMeanBlock;
-    double *buf = nullptr;
-    RZK_CUDA_TRY(cudaMalloc((void **)&buf, sizeof(double) * (nb + 1)));
+    CallScratch mem;
+    RZK_CUDA_TRY(mem.alloc(sizeof(double) * (nb + 1), st));
+    double *buf = (double *)mem.get();
     mean_kernel<<<nb, kMeanBlock, 0, st>>>(s, recv, n_recv, vpls, n_vpl, seed, n_pairs, buf + 1);
     mean_final_kernel<<<1, 32, 0, st>>>(buf + 1, nb, n_pairs, buf);
     cudaError_t e = cudaMemcpyAsync(h_mean, buf, sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(buf);
     if (e != cudaSuccess) { set_last_cuda_error(e, "mean", __FILE__, __LINE__); return RZK_ERR_CUDA; }
     (void)ctx;
     return RZK_OK;

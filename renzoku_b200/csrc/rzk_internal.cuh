@@ -22,6 +22,33 @@ namespace rzk {
 
 void set_last_cuda_error(cudaError_t e, const char *what, const char *file, int line);
 
+// Device scratch of one call, ordered on the call's stream: taken from a memory pool that the
+// library keeps per device and given back to it, on the same stream, when the object dies.
+// A cudaMalloc and cudaFree pair costs 100-400 us each and waits for the whole device (VPL
+// generation of the 24,000-particle frame: 0.64 of 1.1 ms; clustering 10,000 columns: 1.8 of
+// 2.6 ms; many milliseconds now and then); from the pool it is a few microseconds.  The pool
+// keeps at most kPoolKeep bytes that no call uses, serves any number of threads and streams
+// (the runtime orders reuse across streams), and is emptied when the device's last context is
+// destroyed.
+constexpr unsigned long long kPoolKeep = 256ull << 20;
+class CallScratch {
+public:
+    CallScratch() = default;
+    CallScratch(const CallScratch &) = delete;
+    CallScratch &operator=(const CallScratch &) = delete;
+    ~CallScratch() {
+        if (p_) cudaFreeAsync(p_, st_);
+    }
+    cudaError_t alloc(size_t bytes, cudaStream_t st);   // once per object, on the current device
+    char *get() const { return (char *)p_; }
+
+private:
+    void *p_ = nullptr;
+    cudaStream_t st_ = nullptr;
+};
+void pool_context_created(int device);
+void pool_context_destroyed(int device);
+
 // Device error word bits (written by kernels, read by rzk_context_check).
 enum : uint32_t { ERR_TIMEOUT = 1u, ERR_STACK = 2u, ERR_BOUNDS = 4u };
 

@@ -435,9 +435,9 @@ rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st) {
     const size_t o_idx0 = up(2 * sizeof(float4) * (size_t)n), o_idx1 = o_idx0 + up(sizeof(int) * (size_t)n);
     const size_t o_small = o_idx1 + up(sizeof(int) * (size_t)n), o_l0 = o_small + up(sizeof(Task) * (size_t)n);
     const size_t o_l1 = o_l0 + up(sizeof(Task) * (size_t)max_large), o_cnt = o_l1 + up(sizeof(Task) * (size_t)max_large);
-    char *buf = nullptr;
-    RZK_CUDA_TRY(cudaMalloc((void **)&buf, o_cnt + sizeof(int) * (kMaxLevels + 3)));
-    struct Free { char *p; ~Free() { cudaFree(p); } } guard{buf};
+    CallScratch mem;
+    RZK_CUDA_TRY(mem.alloc(o_cnt + sizeof(int) * (kMaxLevels + 3), st));
+    char *buf = mem.get();
     float4 *box = (float4 *)buf;
     int *idx0 = (int *)(buf + o_idx0), *idx1 = (int *)(buf + o_idx1);
     Task *small = (Task *)(buf + o_small), *large[2] = {(Task *)(buf + o_l0), (Task *)(buf + o_l1)};

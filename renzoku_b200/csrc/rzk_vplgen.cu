@@ -244,9 +244,9 @@ rzk_status launch_vplgen(rzk_scene *sc, uint32_t seed, int n_particles, int max_
     size_t slots_bytes = sizeof(rzk_vpl) * (size_t)n_particles * per;
     size_t scan_bytes = exclusive_scan_tmp_bytes(n_particles);
     size_t bytes = slots_bytes + 2 * sizeof(int) * (size_t)n_particles + scan_bytes + 1024;
-    char *buf = nullptr;
-    RZK_CUDA_TRY(cudaMalloc((void **)&buf, bytes));
-    struct Free { char *p; ~Free() { if (p) cudaFree(p); } } guard{buf};
+    CallScratch mem;
+    RZK_CUDA_TRY(mem.alloc(bytes, st));
+    char *buf = mem.get();
     rzk_vpl *slots = (rzk_vpl *)buf;
     int *counts = (int *)(buf + slots_bytes);
     int *offs = counts + n_particles;
