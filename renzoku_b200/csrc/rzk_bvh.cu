@@ -573,6 +573,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
         } else if (r != RZK_OK) {
             return r;
         }
+        RZK_TRY(build_closest_tree(s, st));
     }
     return RZK_OK;
 }

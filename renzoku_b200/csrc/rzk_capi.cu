@@ -74,11 +74,11 @@ void pool_context_destroyed(int device) {
     if (--d.contexts == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
 }
 
-rzk_status launch_occluded(const DevScene &s, const float *p, const float *q, int n, uint8_t *out,
+rzk_status launch_occluded(const DevScene &s, int depth, const float *p, const float *q, int n, uint8_t *out,
                            cudaStream_t st);
 rzk_status launch_ray_query(const DevScene &s, const int *perm, const rzk_ray *rays, int n, int closest,
                             rzk_ray_hit *out, cudaStream_t st);
-rzk_status launch_closest(const DevScene &s, const float *o, const float *d, int n, float *t,
+rzk_status launch_closest(const DevScene &s, int depth, const float *o, const float *d, int n, float *t,
                           rzk_receiver *recv, cudaStream_t st);
 rzk_status launch_primary(const DevScene &s, const rzk_camera &cam, rzk_receiver *out, cudaStream_t st);
 rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, const rzk_receiver *recv,
@@ -190,7 +190,7 @@ static void free_scene(rzk_scene *s) {
                     s->d_bmin, s->d_bmax, s->d_codes, s->d_sorted_codes, s->d_perm, s->d_start,
                     s->d_end, s->d_left, s->d_right, s->d_level, s->d_nbmin, s->d_nbmax,
                     s->d_nodes, s->d_tri_isect, s->d_tri_shade, s->d_surf, s->d_mats,
-                    s->d_lights, s->d_light_pdf, s->d_light_cdf, s->d_wide, s->d_trav};
+                    s->d_lights, s->d_light_pdf, s->d_light_cdf, s->d_wide, s->d_trav, s->d_ctrav};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete s;
@@ -339,14 +339,14 @@ rzk_status rzk_morton_codes(rzk_scene *s, uint32_t *h_codes, void *stream) {
 rzk_status rzk_occluded_batch(rzk_scene *s, const float *d_p, const float *d_q, int n, uint8_t *d_out,
                               void *stream) {
     if (!s || n < 0 || (n > 0 && (!d_p || !d_q || !d_out))) return RZK_ERR_INVALID;
-    return launch_occluded(s->dev(), d_p, d_q, n, d_out, as_stream(stream));
+    return launch_occluded(s->dev(), s->walk_depth(), d_p, d_q, n, d_out, as_stream(stream));
 }
 
 rzk_status rzk_closest_batch(rzk_scene *s, const float *d_o, const float *d_d, int n, float *d_t,
                              rzk_receiver *d_recv, void *stream) {
     if (!s || n < 0 || (n > 0 && (!d_o || !d_d))) return RZK_ERR_INVALID;
     if (d_recv && !aligned16(d_recv)) return RZK_ERR_INVALID;
-    return launch_closest(s->dev(), d_o, d_d, n, d_t, d_recv, as_stream(stream));
+    return launch_closest(s->dev(), s->walk_depth(), d_o, d_d, n, d_t, d_recv, as_stream(stream));
 }
 
 rzk_status rzk_ray_query_batch(rzk_scene *s, const rzk_ray *d_rays, int n, int closest, rzk_ray_hit *d_out,

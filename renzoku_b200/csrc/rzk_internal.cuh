@@ -72,6 +72,9 @@ struct DevScene {
     const float4 *tri_shade;  // 2 x float4 per sorted triangle: {n, surf}, {u, -}
     const float4 *wide;       // 8 x float4 per 4-wide traversal node (see rzk_bvh.cu K6)
     const float4 *trav;       // any-hit tree, same packing as nodes (rzk_sah.cu; = nodes without it)
+    const float4 *ctrav;      // closest-hit tree: trav with inflated boxes (rzk_sah.cu), or null
+    const float *verts;       // 9 per triangle in input order
+    const int *perm;          // sorted triangle slot -> input triangle
     const int4 *surf;         // per surface {mat, flags, light, -}
     const rzk_material *mats;
     const DevLight *lights;
@@ -79,6 +82,7 @@ struct DevScene {
     const float *light_cdf;
     int n_tris, n_nodes, n_mats, n_lights;
     float tmin;
+    float cguard[4];          // origins ctrav covers: centre, squared radius
     uint32_t *err;            // device error word (context-owned)
     unsigned long long *rays; // shadow rays traced by the gather kernels (context-owned counter)
 };
@@ -133,6 +137,9 @@ struct rzk_scene {
     float4 *d_wide = nullptr;
     int n_wide = 0, n_wide_cap = 0;
     float4 *d_trav = nullptr;    // SAH any-hit tree (rzk_sah.cu)
+    float4 *d_ctrav = nullptr;   // closest-hit tree (rzk_sah.cu), not saved: made from d_trav
+    size_t ctrav_bytes = 0;
+    float cguard[4] = {0, 0, 0, -1};
     int trav_depth = 0;
     size_t trav_bytes = 0;
     bool build_trav = true;
@@ -142,11 +149,18 @@ struct rzk_scene {
     float *d_light_pdf = nullptr, *d_light_cdf = nullptr;
     std::vector<int> light_surf;   // host: surface index of each light
     size_t device_bytes = 0;
+    // most entries a walk of the any-hit or closest-hit tree pushes (the reference tree's own
+    // limit where there is neither)
+    int walk_depth() const { return d_trav && trav_depth > 0 ? trav_depth : rzk::STACK_CAP; }
     // scratch for the build (freed after)
     rzk::DevScene dev() const {
         rzk::DevScene s;
         s.nodes = d_nodes; s.tri_isect = d_tri_isect; s.tri_shade = d_tri_shade; s.wide = d_wide;
         s.trav = d_trav ? d_trav : d_nodes;
+        s.ctrav = d_ctrav;
+        for (int i = 0; i < 4; ++i) s.cguard[i] = cguard[i];
+        s.verts = d_v;
+        s.perm = d_perm;
         s.surf = d_surf; s.mats = d_mats; s.lights = d_lights; s.light_pdf = d_light_pdf;
         s.light_cdf = d_light_cdf; s.n_tris = n_tris; s.n_nodes = n_nodes; s.n_mats = n_mats;
         s.n_lights = n_lights; s.tmin = tmin; s.err = ctx ? ctx->d_err : nullptr;
@@ -160,6 +174,7 @@ namespace rzk {
 rzk_status bvh_build(rzk_scene *s, cudaStream_t st);
 // rzk_sah.cu
 rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st);
+rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st);
 // utilities (rzk_bvh.cu)
 rzk_status exclusive_scan_i32(const int *d_in, int *d_out, int n, int *d_total, void *d_tmp,
                               size_t tmp_bytes, cudaStream_t st);

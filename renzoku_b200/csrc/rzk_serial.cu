@@ -189,6 +189,7 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
     rzk_scene *s = new rzk_scene();
     auto fail = [&](rzk_status e) {
         free_arrays(s);
+        if (s->d_ctrav) cudaFree(s->d_ctrav);
         delete s;
         return e;
     };
@@ -254,6 +255,8 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
     }
     for (void **p : {(void **)&s->d_v, (void **)&s->d_tp, (void **)&s->d_tri_surf})
         if (!*p && (e = cudaMalloc(p, 16)) != cudaSuccess) return fail(RZK_ERR_NOMEM);
+    const rzk_status r = build_closest_tree(s, st);
+    if (r != RZK_OK) return fail(r);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) {
         set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
         return fail(RZK_ERR_CUDA);

@@ -1,49 +1,127 @@
 // rzk_trace.cu - batched visibility and closest-hit queries (the Aggregate interface).
 #include "rzk_traverse.cuh"
 
+#include <algorithm>
+
 namespace rzk {
 
 namespace {
 
 constexpr int kTraceBlock = 128;
 
+// The batched queries keep their lanes busy by refilling them: a warp owns a run of rays, and
+// when kRefill of its lanes have finished theirs they take the next ones together, while the
+// others go on.  One ray per thread left 6.7 (closest) and 8.4 (any hit) of 32 lanes active on
+// average, each warp waiting for its longest ray.  The traversal stack has as many entries as
+// the tree walked is deep, so that it does not limit the resident warps (64 entries: 24 per SM).
+constexpr int kRefill = 8;
+
+struct RayRun {   // the warp's rays [next, end)
+    int next, end;
+    __device__ __forceinline__ RayRun(int n, int per_warp) {
+        const long long w = ((long long)blockIdx.x * kTraceBlock + threadIdx.x) >> 5;
+        next = (int)min((long long)n, w * per_warp);
+        end = (int)min((long long)n, w * per_warp + per_warp);
+    }
+    // hands the idle lanes (idx < 0) their next rays' indices; false when the run is over
+    __device__ __forceinline__ bool refill(int &idx, int lane) {
+        const unsigned idle = __ballot_sync(0xffffffffu, idx < 0);
+        if (idle == 0xffffffffu && next >= end) return false;
+        if (next < end && (__popc(idle) >= kRefill)) {
+            const int k = next + __popc(idle & ((1u << lane) - 1u));
+            if (idx < 0 && k < end) idx = k;
+            next += __popc(idle);
+        }
+        return true;
+    }
+};
+
 // Aggregate::hit(p, q, tmin, time) (aggregate.cc:84-90): Ray(p, q - p) over
 // [tmin, |q - p| - tmin].
-__global__ void __launch_bounds__(kTraceBlock) occluded_kernel(DevScene s, const float *p,
-                                                               const float *q, int n,
-                                                               uint8_t *out) {
-    __shared__ int stack_mem[STACK_CAP * kTraceBlock];
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Stack<kTraceBlock> stk;
-    stk.init(stack_mem + threadIdx.x);
-    V3 a = ld3(p + 3 * i), b = ld3(q + 3 * i);
-    Ray r = make_ray(a, sub(b, a));
-    float tmax = len(sub(b, a)) - s.tmin;
-    out[i] = any_hit<kTraceBlock, false, true>(s, r, s.tmin, tmax, stk) ? 1 : 0;
+__global__ void __launch_bounds__(kTraceBlock) occluded_kernel(DevScene s, const float *p, const float *q, int n,
+                                                               int per_warp, int cap, uint8_t *out) {
+    extern __shared__ int stack_mem[];
+    const int lane = threadIdx.x & 31;
+    RayRun run(n, per_warp);
+    AnyHitWalk<kTraceBlock> walk;
+    walk.stk.init(stack_mem + threadIdx.x, cap);
+    int idx = -1;
+    for (;;) {
+        const int was = idx;
+        if (!run.refill(idx, lane)) break;
+        if (idx != was) {
+            const V3 a = ld3(p + 3 * (size_t)idx), b = ld3(q + 3 * (size_t)idx);
+            walk.start(s, make_ray(a, sub(b, a)), s.tmin, len(sub(b, a)) - s.tmin);
+        }
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            if (idx < 0) break;
+            if (walk.step(s)) {
+                out[idx] = walk.hit ? 1 : 0;
+                idx = -1;
+            }
+        }
+    }
 }
 
-__global__ void __launch_bounds__(kTraceBlock) closest_kernel(DevScene s, const float *o,
-                                                              const float *d, int n, float *t_out,
-                                                              rzk_receiver *recv) {
+// One ray per thread, for scenes without a closest-hit tree.
+__global__ void __launch_bounds__(kTraceBlock) closest_plain_kernel(DevScene s, const float *o, const float *d, int n,
+                                                                    float *t_out, rzk_receiver *recv) {
     __shared__ int stack_mem[STACK_CAP * kTraceBlock];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     Stack<kTraceBlock> stk;
     stk.init(stack_mem + threadIdx.x);
-    Ray r = make_ray(ld3(o + 3 * i), ld3(d + 3 * i));
+    Ray r = make_ray(ld3(o + 3 * (size_t)i), ld3(d + 3 * (size_t)i));
     float t, b, g;
-    int slot = closest_hit<kTraceBlock>(s, r, s.tmin, RAY_TMAX, stk, &t, &b, &g);
+    const int slot = closest_hit<kTraceBlock>(s, r, s.tmin, RAY_TMAX, stk, &t, &b, &g);
+    if (t_out) t_out[i] = slot < 0 ? -1.0f : t;
+    if (!recv) return;
     if (slot < 0) {
-        if (t_out) t_out[i] = -1.0f;
-        if (recv) write_miss(recv + i);
+        write_miss(recv + i);
         return;
     }
-    if (t_out) t_out[i] = t;
-    if (recv) {
-        HitGeo h;
-        fill_hit(s, r, slot, t, b, g, h);
-        write_receiver(h, r, recv + i);
+    HitGeo h;
+    fill_hit(s, r, slot, t, b, g, h);
+    write_receiver(h, r, recv + i);
+}
+
+__global__ void __launch_bounds__(kTraceBlock) closest_kernel(DevScene s, const float *o, const float *d, int n,
+                                                              int per_warp, int cap, float *t_out,
+                                                              rzk_receiver *recv) {
+    extern __shared__ int stack_mem[];
+    const int lane = threadIdx.x & 31;
+    RayRun run(n, per_warp);
+    ClosestWalk<kTraceBlock> walk;
+    walk.stk.init(stack_mem + threadIdx.x, cap);
+    int idx = -1, done = -1;   // done: a finished ray whose result is not written yet
+    for (;;) {
+        const int was = idx;
+        const bool more = run.refill(idx, lane);
+        if (done >= 0 && (!more || idx != was)) {
+            int mem[STACK_CAP];   // rarely needed: local memory
+            const int slot = walk.template finish<1>(s, mem);
+            if (t_out) t_out[done] = slot < 0 ? -1.0f : walk.bt;
+            if (recv && slot < 0) {
+                write_miss(recv + done);
+            } else if (recv) {
+                HitGeo h;
+                fill_hit(s, walk.r, slot, walk.bt, walk.bb, walk.bg, h);
+                write_receiver(h, walk.r, recv + done);
+            }
+            done = -1;
+        }
+        if (!more) break;
+        if (idx != was)
+            walk.start(s, make_ray(ld3(o + 3 * (size_t)idx), ld3(d + 3 * (size_t)idx)), s.tmin, RAY_TMAX);
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            if (idx < 0) break;
+            if (walk.step(s)) {
+                done = idx;
+                idx = -1;
+            }
+        }
     }
 }
 
@@ -66,17 +144,18 @@ __global__ void __launch_bounds__(kTraceBlock) ray_query_kernel(DevScene s, cons
     r.org_inv_d = ld3(q.org_inv_d);
     rzk_ray_hit h{0, 0.0f, 0.0f, 0.0f, -1, {0, 0, 0}};
     if (closest) {
-        float t, b, g;
-        const int slot = closest_hit<kTraceBlock>(s, r, q.tmin, q.tmax, stk, &t, &b, &g);
-        if (slot >= 0) {
-            h.hit = 1;
-            h.t = t;
-            h.beta = b;
-            h.gamma = g;
-            h.tri = perm[slot];
+        if (s.n_nodes > 0) {
+            const ClosestHit c = closest_reference<kTraceBlock>(s.nodes, s.tri_isect, s.err, r, q.tmin, q.tmax, stk.base);
+            if (c.slot >= 0) {
+                h.hit = 1;
+                h.t = c.t;
+                h.beta = c.beta;
+                h.gamma = c.gamma;
+                h.tri = perm[c.slot];
+            }
         }
     } else {
-        h.hit = any_hit<kTraceBlock, false, true>(s, r, q.tmin, q.tmax, stk) ? 1 : 0;
+        h.hit = any_hit<kTraceBlock, false, true, false>(s, r, q.tmin, q.tmax, stk) ? 1 : 0;
     }
     out[i] = h;
 }
@@ -103,18 +182,50 @@ __global__ void __launch_bounds__(kTraceBlock) primary_kernel(DevScene s, rzk_ca
 
 }  // namespace
 
-rzk_status launch_occluded(const DevScene &s, const float *p, const float *q, int n, uint8_t *out,
+// Grid of a refilling kernel: one run of at least 32 rays per resident warp, at most kMaxRun.
+struct RunGrid {
+    unsigned blocks;
+    int per_warp, cap;
+    size_t smem;
+};
+template <class K>
+static cudaError_t run_grid(K kernel, int n, int depth, RunGrid &g) {
+    constexpr int kMaxRun = 512;
+    g.cap = std::max(2, std::min(STACK_CAP, depth + 1));
+    g.smem = sizeof(int) * kTraceBlock * (size_t)g.cap;
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTraceBlock, g.smem);
+    if (e != cudaSuccess) return e;
+    const long long warps = (long long)sms * std::max(1, per_sm) * (kTraceBlock / 32);
+    g.per_warp = (int)std::min<long long>(kMaxRun, (n / warps + 31) / 32 * 32 + 32);
+    const long long runs = ((long long)n + g.per_warp - 1) / g.per_warp;
+    g.blocks = (unsigned)((runs + kTraceBlock / 32 - 1) / (kTraceBlock / 32));
+    return cudaSuccess;
+}
+
+rzk_status launch_occluded(const DevScene &s, int depth, const float *p, const float *q, int n, uint8_t *out,
                            cudaStream_t st) {
     if (n <= 0) return RZK_OK;
-    occluded_kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, p, q, n, out);
+    RunGrid g;
+    RZK_CUDA_TRY(run_grid(occluded_kernel, n, depth, g));
+    occluded_kernel<<<g.blocks, kTraceBlock, g.smem, st>>>(s, p, q, n, g.per_warp, g.cap, out);
     RZK_CUDA_TRY(cudaGetLastError());
     return RZK_OK;
 }
 
-rzk_status launch_closest(const DevScene &s, const float *o, const float *d, int n, float *t,
+rzk_status launch_closest(const DevScene &s, int depth, const float *o, const float *d, int n, float *t,
                           rzk_receiver *recv, cudaStream_t st) {
     if (n <= 0) return RZK_OK;
-    closest_kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, o, d, n, t, recv);
+    if (!s.ctrav) {
+        closest_plain_kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, o, d, n, t, recv);
+        RZK_CUDA_TRY(cudaGetLastError());
+        return RZK_OK;
+    }
+    RunGrid g;
+    RZK_CUDA_TRY(run_grid(closest_kernel, n, depth, g));
+    closest_kernel<<<g.blocks, kTraceBlock, g.smem, st>>>(s, o, d, n, g.per_warp, g.cap, t, recv);
     RZK_CUDA_TRY(cudaGetLastError());
     return RZK_OK;
 }

@@ -6,13 +6,15 @@
 // The stack holds these `a` codes, so popping an inner node costs a single 64-byte load
 // that yields both child boxes and both children's own codes.
 //
-// Closest hit visits nodes in exactly the reference's order (aggregate_bvh.cc:402-448):
-// pop, leaf -> triangle test that shrinks tmax, inner -> test left box then right box
-// with the current tmax, push the ones that pass (right is popped first); the loops here
-// go straight on to the entry that would be popped next instead of pushing and popping it.  Any-hit
+// Closest hit gives the reference's answer (aggregate_bvh.cc:402-448: pop, leaf -> triangle
+// test that shrinks tmax, inner -> test left box then right box with the current tmax, push the
+// ones that pass, right popped first) in one of two ways: a nearer-child-first walk of the
+// closest-hit tree wherever that provably finds the same triangle, else the reference's own
+// visit order on the reference tree; see closest_hit below.  Any-hit
 // (aggregate_bvh.cc:452-478) returns whether any reachable triangle passes; its answer
 // does not depend on visit order, so leaf children are tested as soon as their box
-// passes instead of being pushed.  Both keep the reference's 64-entry stack, which drops
+// passes instead of being pushed.  The loops go straight on to the entry that would be popped
+// next instead of pushing and popping it.  All keep the reference's 64-entry stack, which drops
 // pushes when full (holding one entry fewer per level than the reference's, it fills
 // later); a drop sets ERR_STACK in the scene's error word.
 #pragma once
@@ -26,12 +28,12 @@ namespace rzk {
 template <int STRIDE>
 struct Stack {
     int *base;
-    int top;
-    __device__ __forceinline__ void init(int *b) { base = b; top = -1; }
+    int top, cap;
+    __device__ __forceinline__ void init(int *b, int entries = STACK_CAP) { base = b; top = -1; cap = entries; }
     __device__ __forceinline__ bool empty() const { return top < 0; }
     __device__ __forceinline__ int pop() { return base[(top--) * STRIDE]; }
     __device__ __forceinline__ bool push(int v) {
-        if (top < STACK_CAP - 1) { base[(++top) * STRIDE] = v; return true; }
+        if (top < cap - 1) { base[(++top) * STRIDE] = v; return true; }
         return false;
     }
 };
@@ -46,9 +48,25 @@ __device__ __forceinline__ void load_tri(const DevScene &s, int slot, float4 &a,
     a = __ldg(p); b = __ldg(p + 1); c = __ldg(p + 2);
 }
 
+// A pair of sibling nodes: two 32-byte loads (the record is 64-byte aligned).
+__device__ __forceinline__ void load_node(const float4 *p, float4 &a, float4 &b) {
+    uint64_t q[4];
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(q[0]), "=l"(q[1]), "=l"(q[2]), "=l"(q[3]) : "l"(p));
+    auto lo = [](uint64_t x) { return __uint_as_float((uint32_t)x); };
+    auto hi = [](uint64_t x) { return __uint_as_float((uint32_t)(x >> 32)); };
+    a = make_float4(lo(q[0]), hi(q[0]), lo(q[1]), hi(q[1]));
+    b = make_float4(lo(q[2]), hi(q[2]), lo(q[3]), hi(q[3]));
+}
+__device__ __forceinline__ void load_pair(const float4 *p, float4 &l0, float4 &l1, float4 &r0, float4 &r1) {
+    load_node(p, l0, l1);
+    load_node(p + 2, r0, r1);
+}
+
 // TRAV: walk the any-hit tree (DevScene::trav) instead of the reference tree; the answer is
-// the same (see rzk_sah.cu), only the visit order differs.
-template <int STRIDE, bool STATS, bool TRAV = false>
+// the same (see rzk_sah.cu), only the visit order differs.  FASTBOX: the ray was made by
+// make_ray, so box_hit_fast applies (1,000,003 segments on 300k triangles 571 -> 517 us, B200);
+// a caller's own ray may hold any reciprocals and takes box_hit.
+template <int STRIDE, bool STATS, bool TRAV = false, bool FASTBOX = true>
 __device__ __forceinline__ bool any_hit(const DevScene &s, const Ray &r, float tmin, float tmax,
                                         Stack<STRIDE> &stk, TraceStats *ts = nullptr) {
     if (s.n_nodes == 0) return false;
@@ -71,9 +89,11 @@ __device__ __forceinline__ bool any_hit(const DevScene &s, const Ray &r, float t
     for (;;) {
         if (STATS) ts->inner++;
         const float4 *p = tree + 2 * (c + 1);
-        float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
-        bool hl = box_hit(l0, l1, r, tmin, tmax);
-        bool hr = box_hit(r0, r1, r, tmin, tmax);
+        float4 l0, l1, r0, r1;
+        load_pair(p, l0, l1, r0, r1);
+        float tl, tr;
+        bool hl = FASTBOX ? box_hit_fast(l0, l1, r, tmin, tmax, tl) : box_hit(l0, l1, r, tmin, tmax);
+        bool hr = FASTBOX ? box_hit_fast(r0, r1, r, tmin, tmax, tr) : box_hit(r0, r1, r, tmin, tmax);
         int al = __float_as_int(l0.w), ar = __float_as_int(r0.w);
         if (hl && al < 0) {
             if (STATS) ts->leaf++;
@@ -100,38 +120,98 @@ __device__ __forceinline__ bool any_hit(const DevScene &s, const Ray &r, float t
     return false;
 }
 
-// Returns the sorted triangle slot of the closest hit or -1.
+// any_hit on the any-hit tree (TRAV, FASTBOX), one pair of nodes per step.
 template <int STRIDE>
-__device__ __forceinline__ int closest_hit(const DevScene &s, const Ray &r, float tmin, float tmax,
-                                           Stack<STRIDE> &stk, float *t_out, float *beta_out,
-                                           float *gamma_out) {
-    if (s.n_nodes == 0) return -1;
-    float4 lo = __ldg(s.nodes + 2), hi = __ldg(s.nodes + 3);
-    if (!box_hit(lo, hi, r, tmin, tmax)) return -1;
-    int best = -1;
-    float bt = RAY_TMAX, bb = 0.0f, bg = 0.0f;
+struct AnyHitWalk {
+    Stack<STRIDE> stk;
+    Ray r;
+    float tmin, tmax;
+    int c;
+    bool hit, over;
+    __device__ __forceinline__ void start(const DevScene &s, const Ray &ray, float t0, float t1) {
+        r = ray;
+        tmin = t0;
+        tmax = t1;
+        hit = false;
+        over = s.n_nodes == 0;
+        stk.top = -1;
+        c = 0;
+        if (over) return;
+        const float4 lo = __ldg(s.trav + 2), hi = __ldg(s.trav + 3);
+        over = !box_hit(lo, hi, r, tmin, tmax);
+        c = __float_as_int(lo.w);
+        if (!over && c < 0) {
+            hit = tri(s, c);
+            over = true;
+        }
+    }
+    __device__ __forceinline__ bool tri(const DevScene &s, int code) const {
+        float4 ta, tb, tc;
+        load_tri(s, -1 - code, ta, tb, tc);
+        return tri_hit<false>(ta, tb, tc, r, tmin, tmax, nullptr, nullptr, nullptr);
+    }
+    __device__ __forceinline__ bool step(const DevScene &s) {   // true when the walk is over
+        if (over) return true;
+        float4 l0, l1, r0, r1;
+        load_pair(s.trav + 2 * (c + 1), l0, l1, r0, r1);
+        float tl, tr;
+        const bool hl = box_hit_fast(l0, l1, r, tmin, tmax, tl);
+        const bool hr = box_hit_fast(r0, r1, r, tmin, tmax, tr);
+        const int al = __float_as_int(l0.w), ar = __float_as_int(r0.w);
+        if (hl && al < 0) hit = tri(s, al);
+        if (!hit && hr && ar < 0) hit = tri(s, ar);
+        if (hit) return true;
+        const bool gl = hl && al >= 0, gr = hr && ar >= 0;
+        if (gr) {
+            if (gl && !stk.push(al) && s.err) atomicOr(s.err, ERR_STACK);
+            c = ar;
+        } else if (gl) {
+            c = al;
+        } else {
+            if (stk.empty()) return true;
+            c = stk.pop();
+        }
+        return false;
+    }
+};
+
+struct ClosestHit {
+    int slot;   // sorted triangle slot, -1: none
+    float t, beta, gamma;
+};
+
+// The reference's query: its tree, its visit order, its box test, its 64-entry stack (`stack` as
+// Stack::base).  A function of its own, so that a kernel's registers are those of closest_hit's
+// first walk.
+template <int STRIDE>
+__device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const float4 *tri_isect, uint32_t *err,
+                                                     Ray r, float tmin, float tmax, int *stack) {
+    ClosestHit h{-1, RAY_TMAX, 0.0f, 0.0f};
+    float4 lo = __ldg(nodes + 2), hi = __ldg(nodes + 3);
+    if (!box_hit(lo, hi, r, tmin, tmax)) return h;
     bool overflow = false;
-    // as any_hit: the loop continues into the entry it would pop next (the right child
-    // where both boxes pass, each tested with the tmax of that moment) and pushes only the
-    // other, so the nodes are visited in the reference's order
-    stk.top = -1;
+    // the loop continues into the entry it would pop next (the right child where both boxes
+    // pass, each tested with the tmax of that moment) and pushes only the other, so the nodes
+    // are visited in the reference's order
+    Stack<STRIDE> stk;
+    stk.init(stack);
     int c = __float_as_int(lo.w);
     for (;;) {
         if (c < 0) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - c, ta, tb, tc);
+            const float4 *p = tri_isect + 3 * (size_t)(-1 - c);
             float t, b, g;
-            if (tri_hit<true>(ta, tb, tc, r, tmin, tmax, &t, &b, &g)) {
+            if (tri_hit<true>(__ldg(p), __ldg(p + 1), __ldg(p + 2), r, tmin, tmax, &t, &b, &g)) {
                 tmax = t;
-                bt = t; bb = b; bg = g;
-                best = -1 - c;
+                h.t = t; h.beta = b; h.gamma = g;
+                h.slot = -1 - c;
             }
             if (stk.empty()) break;
             c = stk.pop();
             continue;
         }
-        const float4 *p = s.nodes + 2 * (c + 1);
-        float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
+        const float4 *p = nodes + 2 * (c + 1);
+        float4 l0, l1, r0, r1;
+        load_pair(p, l0, l1, r0, r1);
         const bool hl = box_hit(l0, l1, r, tmin, tmax);
         const bool hr = box_hit(r0, r1, r, tmin, tmax);
         if (hr) {
@@ -144,9 +224,129 @@ __device__ __forceinline__ int closest_hit(const DevScene &s, const Ray &r, floa
             c = stk.pop();
         }
     }
-    if (overflow && s.err) atomicOr(s.err, ERR_STACK);
-    if (best >= 0) { *t_out = bt; *beta_out = bb; *gamma_out = bg; }
-    return best;
+    if (overflow && err) atomicOr(err, ERR_STACK);
+    return h;
+}
+
+// The closest hit of a ray made by make_ray over [tmin, tmax]: the sorted triangle slot or -1.
+//
+// Let S be the triangles whose own box passes the slab test over [tmin, tmax] and whose
+// triangle test gives a distance t_k in it; b_k is the box's entry distance.  The reference
+// accepts a triangle of S when it comes to it with max(t_k, b_k) <= its current tmax (boxes
+// above it have smaller entries) and then sets tmax = t_k.  So if some w in S has
+// t_k > L = max(t_w, b_w) for every other k, the reference returns w whatever its order: until
+// it comes to w its tmax stays above L, so w's boxes pass and w is accepted; after that no k is.
+//
+// The walk below looks for w nearer child first.  Its bound is the L of the nearest triangle so
+// far, and it skips only nodes that enter after the bound; the boxes of the closest-hit tree
+// are inflated (rzk_sah.cu) so far that a triangle of S never has a distance below the entry of
+// a box it lies in, whatever the rounding of either test.  So every triangle of S with
+// t_k <= L is met (one skipped under an earlier bound lies beyond that bound's own triangle,
+// which is then a witness itself), and the second distance met tells whether w stands alone.
+// Where it does not (equal distances, shared edges), where the inflation does not cover the ray
+// (closest_covered) or the scene has no such tree, the reference's own order decides.
+// 524,288 scattered rays on 300k triangles, one per thread: 1,350 us in the reference's order, 590
+// here; with the lanes refilled 433 us (B200).  Rays of the rooms here need the reference's own
+// order about once in 1,000 (primary hits) to never (scattered rays).
+__device__ __forceinline__ bool closest_covered(const DevScene &s, const Ray &r) {
+    const V3 q = sub(r.o, ld3(s.cguard));
+    return s.ctrav != nullptr && dot(q, q) <= s.cguard[3];   // no for a NaN
+}
+
+// The slab test of a sorted triangle's own box, formed from its vertices as the build forms it.
+__device__ __forceinline__ bool own_box_hit(const DevScene &s, int slot, const Ray &r, float tmin, float tmax,
+                                            float &enter) {
+    const float *v = s.verts + 9 * (size_t)__ldg(s.perm + slot);
+    const V3 p0 = mk(__ldg(v), __ldg(v + 1), __ldg(v + 2)), p1 = mk(__ldg(v + 3), __ldg(v + 4), __ldg(v + 5)),
+             p2 = mk(__ldg(v + 6), __ldg(v + 7), __ldg(v + 8));
+    const V3 lo = vmin(vmin(p0, p1), p2), hi = vmax(vmax(p0, p1), p2);
+    return box_hit_fast(make_float4(lo.x, lo.y, lo.z, 0.0f), make_float4(hi.x, hi.y, hi.z, 0.0f), r, tmin, tmax, enter);
+}
+
+// The walk, one node or leaf per step, for kernels that refill their lanes between steps.
+template <int STRIDE>
+struct ClosestWalk {
+    Stack<STRIDE> stk;
+    Ray r;
+    float tmin, tmax, bound, bt, lim, bb, bg, second;
+    int c, best;
+    bool sure;
+    __device__ __forceinline__ void start(const DevScene &s, const Ray &ray, float t0, float t1) {
+        r = ray;
+        tmin = t0;
+        tmax = bound = bt = t1;
+        lim = t0;
+        bb = bg = 0.0f;
+        second = INFINITY;
+        best = -1;
+        stk.top = -1;
+        sure = s.n_nodes > 0 && closest_covered(s, r);
+        c = sure ? __float_as_int(__ldg(&s.ctrav[2].w)) : 0;
+    }
+    // true when the walk is over (finish() has the answer)
+    __device__ __forceinline__ bool step(const DevScene &s) {
+        if (!sure) return true;
+        if (c < 0) {
+            float4 ta, tb, tc;
+            load_tri(s, -1 - c, ta, tb, tc);
+            float t, b, g, enter = 0.0f;
+            if (tri_hit<true>(ta, tb, tc, r, tmin, bound, &t, &b, &g) && own_box_hit(s, -1 - c, r, tmin, tmax, enter)) {
+                if (t < bt || best < 0) {
+                    if (best >= 0) second = fminf(second, bt);
+                    best = -1 - c;
+                    bt = t; bb = b; bg = g;
+                    lim = enter;
+                    bound = fmaxf(t, enter);
+                } else {
+                    second = fminf(second, t);
+                }
+            }
+            if (stk.empty()) return true;
+            c = stk.pop();
+            return false;
+        }
+        float4 l0, l1, r0, r1;
+        load_pair(s.ctrav + 2 * (c + 1), l0, l1, r0, r1);
+        float tl, tr;
+        const bool hl = box_hit_fast(l0, l1, r, tmin, bound, tl);
+        const bool hr = box_hit_fast(r0, r1, r, tmin, bound, tr);
+        if (hl && hr) {
+            const bool lf = tl <= tr;
+            if (!stk.push(__float_as_int(lf ? r0.w : l0.w))) sure = false;   // not met: as deep as the tree
+            c = __float_as_int(lf ? l0.w : r0.w);
+        } else if (hl || hr) {
+            c = __float_as_int(hl ? l0.w : r0.w);
+        } else {
+            if (stk.empty()) return true;
+            c = stk.pop();
+        }
+        return false;
+    }
+    // the answer; `stack`: room for the reference's own walk, STACK_CAP entries STRIDE2 apart
+    template <int STRIDE2>
+    __device__ __forceinline__ int finish(const DevScene &s, int *stack) {
+        if (s.n_nodes == 0) return -1;
+        if (!sure || (best >= 0 && second <= fmaxf(bt, lim))) {
+            const ClosestHit h = closest_reference<STRIDE2>(s.nodes, s.tri_isect, s.err, r, tmin, tmax, stack);
+            best = h.slot;
+            bt = h.t; bb = h.beta; bg = h.gamma;
+        }
+        return best;
+    }
+};
+
+// stk: STACK_CAP entries
+template <int STRIDE>
+__device__ __forceinline__ int closest_hit(const DevScene &s, const Ray &r, float tmin, float tmax,
+                                           Stack<STRIDE> &stk, float *t_out, float *beta_out,
+                                           float *gamma_out) {
+    ClosestWalk<STRIDE> w;
+    w.stk = stk;
+    w.start(s, r, tmin, tmax);
+    while (!w.step(s)) {}
+    const int slot = w.template finish<STRIDE>(s, stk.base);
+    if (slot >= 0) { *t_out = w.bt; *beta_out = w.bb; *gamma_out = w.bg; }
+    return slot;
 }
 
 struct HitGeo {
