@@ -499,6 +499,98 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_persistent_kernel(
     }
 }
 
+// The gather in two passes.  A receiver's sum over a chunk has one order, so in one pass an item
+// is a tile and a whole chunk (128 VPLs or more): milliseconds of one warp's serial work, and
+// below some billions of pairs the launch lasts as long as its longest items.  In two passes the
+// shadow rays run as items of few VPLs, each leaving one visibility ballot per VPL, and a block
+// per (tile, chunk) then forms the marked pairs' terms in parallel and adds them in VPL order -
+// the same terms in the same order (two_pass_group says where this pays).
+template <int WARPS, int TILE, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) gather_vis_kernel(DevScene s, const rzk_receiver *recv, int n_recv,
+                                                                      int img_w, const rzk_vpl *vpls, int n_vpl,
+                                                                      int group, int n_groups, int n_wtiles, int *work,
+                                                                      uint32_t *masks) {
+    __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
+    __shared__ __align__(8) uint64_t bar[WARPS][2];
+    __shared__ int stacks[WARPS][STACK_CAP];
+
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    WarpStage<TILE> ws;
+    ws.init(tiles[w], bar[w], stacks[w], lane);
+    const long long n_items = (long long)n_wtiles * n_groups;
+    while (true) {
+        int item = 0;
+        if (lane == 0) item = atomicAdd(work, 1);
+        item = __shfl_sync(kFull, item, 0);
+        if (item >= n_items) break;
+        const int wt = item / n_groups;
+        const int j0 = (item - wt * n_groups) * group, j1 = min(n_vpl, j0 + group);
+        if (!visibility_item<TILE>(s, recv, n_recv, img_w, vpls, j0, j1, wt, ws, lane,
+                                   masks + (size_t)wt * n_vpl + j0))
+            break;
+    }
+}
+
+// One warp per (tile, chunk), where there are enough of them: no exchange between warps.
+constexpr int kShadeBlock = 128;
+__global__ void __launch_bounds__(kShadeBlock) gather_shade_kernel(DevScene s, const rzk_receiver *recv, int n_recv,
+                                                                   int img_w, const rzk_vpl *vpls, int n_vpl,
+                                                                   int chunk_len, int n_chunks, long long n_items,
+                                                                   const uint32_t *masks, int mode, float tau,
+                                                                   float *partial) {
+    const long long item = ((long long)blockIdx.x * kShadeBlock + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (item >= n_items) return;
+    const int wt = (int)(item / n_chunks), chunk = (int)(item - (long long)wt * n_chunks);
+    const int ri = lane_receiver(wt, lane, n_recv, img_w);
+    RecvRegs r;
+    rzk_material rm;
+    bool active = false;
+    if (ri >= 0) {
+        r = load_receiver(recv + ri);
+        active = r.mat >= 0;
+        if (active) rm = load_material(s.mats + r.mat);
+    }
+    const int j0 = chunk * chunk_len, j1 = min(n_vpl, j0 + chunk_len);
+    const uint32_t *m = masks + (size_t)wt * n_vpl;
+    Rgb sum = crgb(0.0f, 0.0f, 0.0f);
+    for (int b = j0; b < j1; b += 32) {
+        const uint32_t word = b + lane < j1 ? __ldcs(m + b + lane) : 0u;
+        for (unsigned todo = __ballot_sync(kFull, word != 0u); todo; todo &= todo - 1u) {
+            const int v = __ffs(todo) - 1;
+            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
+            const rzk_vpl l = load_vpl(vpls + b + v);
+            sum = cadd(sum, pair_radiance(s, r, rm, l, pair_geo(r, l), mode, tau));
+        }
+    }
+    if (ri >= 0) {
+        float *o = partial + 3 * ((size_t)chunk * n_recv + ri);
+        __stcs(o, sum.r); __stcs(o + 1, sum.g); __stcs(o + 2, sum.b);
+    }
+}
+
+// One block per (tile, chunk) otherwise.
+constexpr int kShadeWarps = 8;
+__global__ void __launch_bounds__(32 * kShadeWarps) gather_shade_block_kernel(DevScene s, const rzk_receiver *recv, int n_recv,
+                                                                        int img_w, const rzk_vpl *vpls, int n_vpl,
+                                                                        int chunk_len, int n_chunks,
+                                                                        const uint32_t *masks, int mode, float tau,
+                                                                        float *partial) {
+    __shared__ float terms[32][3][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int wt = blockIdx.x / n_chunks, chunk = blockIdx.x - wt * n_chunks;
+    const int ri = lane_receiver(wt, lane, n_recv, img_w);
+    RecvRegs r;
+    bool active = false;
+    if (ri >= 0) {
+        r = load_receiver(recv + ri);
+        active = r.mat >= 0;
+    }
+    const int j0 = chunk * chunk_len, j1 = min(n_vpl, j0 + chunk_len);
+    const float sum = shade_chunk<kShadeWarps>(s, r, active, vpls, j0, j1, masks + (size_t)wt * n_vpl + j0, mode, tau, terms);
+    if (w < 3 && ri >= 0) __stcs(partial + 3 * ((size_t)chunk * n_recv + ri) + w, sum);
+}
+
 __global__ void reduce_chunks_kernel(const float *partial, int n_recv, int n_chunks, float scale,
                                      float *out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -675,6 +767,51 @@ __global__ void order_keys_kernel(const __grid_constant__ OrderTable t, uint32_t
     idx[i] = i;
 }
 
+// The order of at most kRankMax VPLs in one launch: a key's place is the number of keys before it
+// (smaller, or equal and earlier).  A block places its keys against all of them, read from shared
+// memory four at a time, and copies its VPLs there.  For a few thousand keys this is faster than
+// the radix sort's ten dependent launches: 333 VPLs 7 us and 36 (with the launches' gaps), 4,096
+// VPLs 22 us and 60; at 8,192 the two are level (the work here is quadratic).
+constexpr int kRankThreads = 64, kRankTile = 1024, kRankMax = 4096;
+__global__ void __launch_bounds__(kRankThreads) order_rank_kernel(const __grid_constant__ OrderTable t,
+                                                                  const uint32_t *keys, rzk_vpl *out) {
+    __shared__ __align__(16) uint32_t sh[kRankTile];
+    __shared__ int place[kRankThreads];
+    const int first = blockIdx.x * kRankThreads, i = first + threadIdx.x;
+    const uint32_t mine = i < t.total ? keys[i] : 0u;
+    int before[4] = {0, 0, 0, 0};
+    for (int b = 0; b < t.total; b += kRankTile) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < kRankTile; k += kRankThreads) sh[k] = b + k < t.total ? keys[b + k] : 0xffffffffu;
+        __syncthreads();
+        // keys of an earlier block's range count when equal, of a later one's not: a limit one
+        // higher turns <= into < (a key has 31 bits at most)
+        auto count = [&](int k0, int k1, uint32_t limit) {
+#pragma unroll 4
+            for (int k = k0; k < k1; k += 4) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(sh + k);
+                before[0] += v.x < limit;
+                before[1] += v.y < limit;
+                before[2] += v.z < limit;
+                before[3] += v.w < limit;
+            }
+        };
+        const int own0 = min(max(first - b, 0), kRankTile), own1 = min(max(first + kRankThreads - b, 0), kRankTile);
+        count(0, own0, mine + 1u);
+        for (int k = own0; k < own1; ++k) before[0] += sh[k] < mine || (sh[k] == mine && b + k < i);
+        count(own1, kRankTile, mine);
+    }
+    place[threadIdx.x] = before[0] + before[1] + before[2] + before[3];
+    __syncthreads();
+    constexpr int W = (int)(sizeof(rzk_vpl) / 16);
+    const int n = min(kRankThreads, t.total - first);
+    for (int e = threadIdx.x; e < n * W; e += kRankThreads) {
+        const int k = e / W, c = e % W;
+        const OrderSeg &g = t.seg[order_seg_of(t, first + k)];
+        reinterpret_cast<float4 *>(out + place[k])[c] = reinterpret_cast<const float4 *>(g.src + (first + k - g.begin))[c];
+    }
+}
+
 // out[j] = concatenated VPL idx[j], one 4-byte word per thread (coalesced writes; each
 // record's 96 bytes are read by 24 consecutive threads).
 __global__ void order_permute_kernel(const __grid_constant__ OrderTable t, const int *idx, rzk_vpl *out) {
@@ -730,6 +867,7 @@ size_t order_scratch_bytes(int total) {
 }
 
 int order_launches(const OrderTable &t) {
+    if (t.total > 0 && t.total <= kRankMax) return 2;
     return t.total > 0 ? 2 + radix_sort_launches(t.total, order_bits(t)) : 0;
 }
 
@@ -741,6 +879,11 @@ rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStre
     void *sort = p + 2 * order_up(sizeof(uint32_t) * (size_t)t.total);
     order_keys_kernel<<<(t.total + 255) / 256, 256, 0, st>>>(t, keys, idx);
     RZK_CUDA_TRY(cudaGetLastError());
+    if (t.total <= kRankMax) {
+        order_rank_kernel<<<(t.total + kRankThreads - 1) / kRankThreads, kRankThreads, 0, st>>>(t, keys, out);
+        RZK_CUDA_TRY(cudaGetLastError());
+        return RZK_OK;
+    }
     RZK_TRY(radix_sort_u32(keys, idx, t.total, order_bits(t), sort, st));
     const long long words = (long long)t.total * (long long)(sizeof(rzk_vpl) / 4);
     order_permute_kernel<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(t, idx, out);
@@ -816,7 +959,7 @@ int gather_launches(int n_recv, int n_vpl, int n_chunks) {
     if (n_recv <= 0) return 0;
     int chunk_len = 0;
     resolve_chunks(n_vpl, n_chunks, chunk_len);
-    int k = 2;   // gather + chunk reduction
+    int k = 3;   // tracing, summing, chunk reduction (one less in one pass)
     if (n_chunks > 1) {
         OrderTable t;
         order_table_init(t);
@@ -825,6 +968,31 @@ int gather_launches(int n_recv, int n_vpl, int n_chunks) {
         k += order_launches(t);
     }
     return k;
+}
+
+// VPLs per tracing item of a two-pass gather, or 0 where one pass does.  Two passes are faster up
+// to some 2e9 pairs (measured to 2.7e8; us, one pass and two, B200): 61 x 47 receivers x 333 VPLs,
+// 36 triangles 657 and 96; 30k triangles 64^2 x 300 5,970 and 494, 128^2 x 3,000 11,400 and 6,850,
+// 256^2 x 3,000 17,900 and 16,300; 300k triangles 128^2 x 8,000 9,800 and 4,700; 36 triangles
+// 256^2 x 4,096 8,080 and 8,110.  At 512^2 x 32,768 (8.6e9 pairs, 300k triangles) they take 106 ms
+// to one pass's 103 and 1.07 GB of ballots.  About twenty items per resident warp even the warps'
+// loads out (3 leave a tail, 60 cost more in cold occluder caches); an item of more than 256 VPLs
+// gains nothing by being longer.
+static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, int &group) {
+    constexpr long long kMaskWords = 64ll << 20;   // 256 MB of ballots
+    constexpr long long kItems = 20, kMaxGroup = 256;
+    group = 0;
+    if (wtiles * n_vpl > kMaskWords) return RZK_OK;
+    if (ctx->vis_grid == 0) {
+        int dev = 0, sms = 0, per_sm = 0;
+        RZK_CUDA_TRY(cudaGetDevice(&dev));
+        RZK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 32, 7>, 128, 0));
+        ctx->vis_grid = std::max(1, sms * std::max(1, per_sm));
+    }
+    group = (int)std::min<long long>(kMaxGroup, std::max<long long>(1, wtiles * n_vpl / (kItems * 4 * ctx->vis_grid)));
+    if (group > 32) group = group / 32 * 32;   // whole shared-memory tiles
+    return RZK_OK;
 }
 
 rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, const rzk_receiver *recv,
@@ -842,7 +1010,10 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     resolve_chunks(n_vpl, n_chunks, chunk_len);
     // one plane of partial sums per chunk, added by reduce_chunks_kernel (the chunk ring that
     // rzk_gather_noalloc sums in measured 1.3% slower here, where memory is not short)
-    const size_t need = sizeof(float) * 3 * (size_t)n_recv * n_chunks;
+    const size_t plane_bytes = (sizeof(float) * 3 * (size_t)n_recv * n_chunks + 255) & ~(size_t)255;
+    int group = 0;
+    if (variant == 0 && n_vpl > 0) RZK_TRY(two_pass_group(ctx, wtiles, n_vpl, group));
+    const size_t need = plane_bytes + (group > 0 ? sizeof(uint32_t) * (size_t)wtiles * n_vpl : 0);
     if (need > ctx->partial_bytes) {
         if (ctx->d_partial) cudaFree(ctx->d_partial);
         ctx->d_partial = nullptr;
@@ -853,7 +1024,22 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     if (!ctx->d_work) RZK_CUDA_TRY(cudaMalloc((void **)&ctx->d_work, 64));
     float *part = ctx->d_partial;
     if (n_chunks > 1) RZK_TRY(order_gather_vpls(ctx, box, vpls, n_vpl, &vpls, st));
-    if (gv.kind == 3) {
+    if (group > 0) {
+        uint32_t *masks = (uint32_t *)((char *)part + plane_bytes);
+        const int n_groups = (n_vpl + group - 1) / group;
+        RZK_CUDA_TRY(cudaMemsetAsync(ctx->d_work, 0, sizeof(int), st));
+        const long long blocks = std::min<long long>(ctx->vis_grid, (wtiles * n_groups + 3) / 4);
+        gather_vis_kernel<4, 32, 7><<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, group, n_groups,
+                                                                      (int)wtiles, ctx->d_work, masks);
+        RZK_CUDA_TRY(cudaGetLastError());
+        const long long items = wtiles * n_chunks;
+        if (items >= 4ll * ctx->vis_grid)
+            gather_shade_kernel<<<(unsigned)((items + 3) / 4), kShadeBlock, 0, st>>>(
+                s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, items, masks, mode, tau, part);
+        else
+            gather_shade_block_kernel<<<(unsigned)items, 32 * kShadeWarps, 0, st>>>(
+                s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, masks, mode, tau, part);
+    } else if (gv.kind == 3) {
         RZK_CUDA_TRY(cudaMemsetAsync(ctx->d_work, 0, sizeof(int), st));
         const int wt = (int)wtiles;
         const ChunkRing nr{};

@@ -72,6 +72,18 @@ __device__ __forceinline__ RecvRegs load_receiver(const rzk_receiver *r) {
     return o;
 }
 
+// A VPL record in registers: six 16-byte loads (the library's VPL arrays are 16-byte aligned).
+__device__ __forceinline__ rzk_vpl load_vpl(const rzk_vpl *v) {
+    union {
+        float4 f[6];
+        rzk_vpl l;
+    } u;
+    static_assert(sizeof(u.f) == sizeof(u.l), "96-byte records");
+#pragma unroll
+    for (int k = 0; k < 6; ++k) u.f[k] = __ldg(reinterpret_cast<const float4 *>(v) + k);
+    return u.l;
+}
+
 // r with its tangent basis vectors u, v read again from the receiver record
 __device__ __forceinline__ RecvRegs reload_basis(RecvRegs r, const rzk_receiver *rec) {
     const float4 *q = reinterpret_cast<const float4 *>(rec);
@@ -137,15 +149,21 @@ __device__ __forceinline__ bool vpl_from_behind(const rzk_vpl &l) {
     return l.mat >= 0 && dot(ld3(l.wi), ld3(l.nn)) <= ZERO_EPSILON;
 }
 
+__device__ __forceinline__ PairGeo pair_geo(const RecvRegs &r, const rzk_vpl &l) {
+    PairGeo pg;
+    pg.q = ld3(l.p);
+    pg.G = form_factor_abs(r.p, r.ns, pg.q, ld3(l.n));
+    pg.wi = unit(sub(pg.q, r.p));
+    pg.power = crgb(l.contrib[0], l.contrib[1], l.contrib[2]);
+    return pg;
+}
+
 // Geometry of a pair and the exact-zero test of its term: returns false when either
 // BRDF's early-out makes the term exactly zero (G and the power finite).  `fin` and
 // `behind` are vpl_power_finite(l) and vpl_from_behind(l).
 __device__ __forceinline__ bool pair_survives(const RecvRegs &r, const rzk_vpl &l, PairGeo &pg, bool fin,
                                               bool behind) {
-    pg.q = ld3(l.p);
-    pg.G = form_factor_abs(r.p, r.ns, pg.q, ld3(l.n));
-    pg.wi = unit(sub(pg.q, r.p));
-    pg.power = crgb(l.contrib[0], l.contrib[1], l.contrib[2]);
+    pg = pair_geo(r, l);
     if (isfinite(pg.G) && fin) {
         if (dot(pg.wi, r.uvn.n) <= ZERO_EPSILON || dot(r.wo, r.uvn.n) <= ZERO_EPSILON) return false;
         if (behind) return false;
@@ -520,25 +538,66 @@ __device__ __forceinline__ bool visibility_item(const DevScene &s, const rzk_rec
         const rzk_vpl &mine = tile[lane < cnt ? lane : 0];
         const unsigned fin_mask = __ballot_sync(kFull, lane < cnt && vpl_power_finite(mine));
         const unsigned behind_mask = __ballot_sync(kFull, lane < cnt && vpl_from_behind(mine));
+        uint32_t word = 0u;   // the ballot of the tile's VPL `lane`
         for (int v = 0; v < cnt; ++v) {
             const rzk_vpl &l = tile[v];
             const bool fin = (fin_mask >> v) & 1u, behind = (behind_mask >> v) & 1u;
+            if (!__any_sync(kFull, active && !pair_clearly_zero(r, l, fin, behind))) continue;
             PairGeo pg;
-            bool act = active && !pair_clearly_zero(r, l, fin, behind) && pair_survives(r, l, pg, fin, behind);
-            unsigned vis = 0u;
+            const bool act = active && pair_survives(r, l, pg, fin, behind);
             const unsigned am = __ballot_sync(kFull, act);
+            if (!am) continue;
             n_rays += (unsigned)__popc(am);
-            if (am) {
-                Ray ray = make_ray(r.p, sub(pg.q, r.p));
-                float tmax = len(sub(pg.q, r.p)) - s.tmin;
-                vis = __ballot_sync(kFull, packet_visible_near(s, ray, tmax, act, ws.stk, occ_cache, occ_cache2));
-            }
-            if (lane == 0) masks[k * TILE + v] = vis;
+            Ray ray = make_ray(r.p, sub(pg.q, r.p));
+            float tmax = len(sub(pg.q, r.p)) - s.tmin;
+            const unsigned vis =
+                __ballot_sync(kFull, packet_visible_near(s, ray, tmax, act, ws.stk, occ_cache, occ_cache2));
+            if (lane == v) word = vis;
         }
+        if (lane < cnt) masks[k * TILE + lane] = word;
         __syncwarp();
     }
     if (lane == 0 && s.rays && n_rays) atomicAdd(s.rays, n_rays);
     return true;
+}
+
+// Summing half with one order of additions per sum but the terms formed in parallel: the warps
+// of a block (at least three) take the VPLs of [j0, j1) in turn, 32 VPLs at a time, and leave the
+// terms in `terms`; then thread t < 96 adds channel t / 32 of receiver t % 32 in VPL order.
+// Returns that thread's sum.  `masks` as from visibility_item, its first word VPL j0's.
+template <int WARPS>
+__device__ __forceinline__ float shade_chunk(const DevScene &s, const RecvRegs &r, bool active, const rzk_vpl *vpls,
+                                             int j0, int j1, const uint32_t *masks, int mode, float tau,
+                                             float (*terms)[3][32]) {
+    static_assert(WARPS >= 3, "a warp per channel");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float acc = 0.0f;
+    for (int b = j0; b < j1; b += 32) {
+        const uint32_t word = b + lane < j1 ? __ldg(masks + (b - j0) + lane) : 0u;
+        const unsigned some = __ballot_sync(kFull, word != 0u);   // the same in every warp
+        if (!some) continue;
+        int k = 0;
+        for (unsigned todo = some; todo; todo &= todo - 1u, ++k) {
+            if (k % WARPS != w) continue;
+            const int v = __ffs(todo) - 1;
+            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
+            const rzk_vpl l = load_vpl(vpls + b + v);
+            const PairGeo pg = pair_geo(r, l);
+            const Rgb L = pair_radiance(s, r, load_material(s.mats + r.mat), l, pg, mode, tau);
+            terms[v][0][lane] = L.r;
+            terms[v][1][lane] = L.g;
+            terms[v][2][lane] = L.b;
+        }
+        __syncthreads();
+        if (w < 3) {
+            for (unsigned todo = some; todo; todo &= todo - 1u) {
+                const int v = __ffs(todo) - 1;
+                if ((__shfl_sync(kFull, word, v) >> lane) & 1u) acc += terms[v][w][lane];
+            }
+        }
+        __syncthreads();
+    }
+    return acc;
 }
 
 // Summing half: the 32 receivers of warp tile `wt` add, in VPL order, the terms of the

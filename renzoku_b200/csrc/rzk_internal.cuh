@@ -110,6 +110,7 @@ struct rzk_context {
     void *d_order = nullptr;
     size_t order_bytes = 0;
     int persistent_grid[16] = {0};
+    int vis_grid = 0;   // resident grid of the two-pass gather's tracing kernel
 };
 
 struct rzk_scene {
