@@ -19,13 +19,15 @@
 namespace rzk {
 
 struct BatchJob {
-    DevScene s;
+    GatherScene s;
     const rzk_receiver *recv;
     const rzk_vpl *vpls;
     float *partial;
     float *out;
     long long item_begin;   // first work item of this job
     long long out_begin;    // first output float (3 per receiver) of this job in the batch
+    long long vis_begin;    // two passes: first tracing item, and first visibility word
+    long long mask_begin;
     int n_recv, img_w, n_vpl, chunk_len, n_chunks, n_wtiles, mode;
     float tau, scale;
 };
@@ -39,20 +41,75 @@ struct JobTable {
     BatchJob jobs[kJobsPerLaunch];
     int n_jobs;
     int n_items;
+    int n_vis;              // two passes: tracing items (0: one pass), VPLs in each
+    int group;
     long long n_out;
+    long long n_words;      // visibility words of the table's jobs
 };
 static_assert(sizeof(JobTable) <= 32000, "kernel parameter block limit");
 
 namespace {
 
-__device__ __forceinline__ int find_job(const JobTable &t, long long item, bool by_out) {
+template <class Begin>
+__device__ __forceinline__ int find_job(const JobTable &t, long long item, Begin begin) {
     int lo = 0, hi = t.n_jobs - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        long long b = by_out ? t.jobs[mid].out_begin : t.jobs[mid].item_begin;
-        if (b <= item) lo = mid; else hi = mid - 1;
+        if (begin(t.jobs[mid]) <= item) lo = mid; else hi = mid - 1;
     }
     return lo;
+}
+__device__ __forceinline__ int job_of_item(const JobTable &t, long long item) {
+    return find_job(t, item, [](const BatchJob &j) { return j.item_begin; });
+}
+
+// The two-pass gather (gather_vis_kernel, gather_shade_kernel in rzk_gather.cu) over the table's
+// jobs: tracing items of t.group VPLs, then a warp per (job, tile, chunk).
+template <int WARPS, int TILE, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) batch_vis_kernel(const __grid_constant__ JobTable t, int *work,
+                                                                     uint32_t *masks) {
+    __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
+    __shared__ __align__(8) uint64_t bar[WARPS][2];
+    __shared__ int stacks[WARPS][STACK_CAP];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    WarpStage<TILE> ws;
+    ws.init(tiles[w], bar[w], stacks[w], lane);
+    while (true) {
+        int item = 0;
+        if (lane == 0) item = atomicAdd(work, 1);
+        item = __shfl_sync(kFull, item, 0);
+        if (item >= t.n_vis) break;
+        const BatchJob &jb = t.jobs[find_job(t, item, [](const BatchJob &j) { return j.vis_begin; })];
+        const int n_groups = (jb.n_vpl + t.group - 1) / t.group;
+        const int local = item - (int)jb.vis_begin;
+        const int wt = local / n_groups;
+        const int j0 = (local - wt * n_groups) * t.group, j1 = min(jb.n_vpl, j0 + t.group);
+        if (!visibility_item<TILE>(jb.s, jb.recv, jb.n_recv, jb.img_w, jb.vpls, j0, j1, wt, ws, lane,
+                                   masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0))
+            break;
+    }
+}
+
+constexpr int kShadeBlock = 128;
+__global__ void __launch_bounds__(kShadeBlock) batch_shade_kernel(const __grid_constant__ JobTable t,
+                                                                  const uint32_t *masks) {
+    const long long item = ((long long)blockIdx.x * kShadeBlock + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (item >= t.n_items) return;
+    const BatchJob &jb = t.jobs[job_of_item(t, item)];
+    const int local = (int)(item - jb.item_begin);
+    const int wt = local / jb.n_chunks, chunk = local - wt * jb.n_chunks;
+    const int ri = lane_receiver(wt, lane, jb.n_recv, jb.img_w);
+    RecvRegs r;
+    rzk_material rm;
+    if (ri >= 0) {
+        r = load_receiver(jb.recv + ri);
+        if (r.mat >= 0) rm = load_material(jb.s.mats + r.mat);
+    }
+    const int j0 = chunk * jb.chunk_len, j1 = min(jb.n_vpl, j0 + jb.chunk_len);
+    const Rgb sum = shade_marked(jb.s, r, rm, jb.vpls, j0, j1, masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0,
+                                 jb.mode, jb.tau, lane);
+    PlaneSink{jb.partial, jb.n_recv, chunk}(ri, sum, true);
 }
 
 template <int WARPS, int TILE, int MINB, int TW = 8>
@@ -69,7 +126,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_gather_kernel(const __
         if (lane == 0) item = atomicAdd(work, 1);
         item = __shfl_sync(kFull, item, 0);
         if (item >= t.n_items) break;
-        const int j = find_job(t, item, false);
+        const int j = job_of_item(t, item);
         const BatchJob &jb = t.jobs[j];
         const int local = item - (int)jb.item_begin;
         const int wt = local / jb.n_chunks;   // tile-major, as gather_persistent_kernel
@@ -83,7 +140,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_gather_kernel(const __
 __global__ void batch_reduce_kernel(const __grid_constant__ JobTable t) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= t.n_out) return;
-    const int j = find_job(t, i, true);
+    const int j = find_job(t, i, [](const BatchJob &b) { return b.out_begin; });
     const BatchJob &jb = t.jobs[j];
     const long long k = i - jb.out_begin;
     const long long stride = 3LL * jb.n_recv;
@@ -139,6 +196,7 @@ struct BatchPlan {
     std::vector<size_t> order_base;          // per table: its first VPL in the sorted copy
     size_t sorted_vpls = 0;
     int max_order_total = 0;
+    int vis_grid = 0;              // resident grid of the two-pass tracing kernel
     size_t partial_floats = 0;
     float *bound = nullptr;        // partial buffer the tables point into
     void *order_bound = nullptr;   // ordering buffer the ordered jobs point into
@@ -206,6 +264,8 @@ rzk_status batch_plan_create(const rzk_gather_job *jobs, int n_jobs, int chunk_l
         }
         JobTable &t = p->tables.back();
         BatchJob &b = h[i];
+        b.mask_begin = t.n_words;
+        t.n_words += (long long)b.n_wtiles * b.n_vpl;
         b.item_begin = t.n_items;
         b.out_begin = t.n_out;
         t.n_items += (int)items;
@@ -225,6 +285,39 @@ rzk_status batch_plan_create(const rzk_gather_job *jobs, int n_jobs, int chunk_l
     return RZK_OK;
 }
 
+// Two passes for a table within the ballots' budget (64 M words, 256 MB), the items as in
+// rzk_gather: about twenty per resident warp.
+constexpr long long kBatchMaskWords = 64ll << 20;
+size_t batch_plan_mask_words(const BatchPlan *p) {
+    long long most = 0;
+    for (const JobTable &t : p->tables)
+        if (t.n_words <= kBatchMaskWords) most = std::max(most, t.n_words);
+    return (size_t)most;
+}
+
+static int vis_grid() {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_vis_kernel<4, 32, 7>, 128, 0);
+    return std::max(1, sms * std::max(1, per_sm));
+}
+
+// Sets the table's tracing items; false where one pass has to do.
+static bool plan_vis(JobTable &t, int grid) {
+    if (t.n_words <= 0 || t.n_words > kBatchMaskWords) return false;
+    long long g = std::min<long long>(256, std::max<long long>(1, t.n_words / (20 * 4 * (long long)grid)));
+    if (g > 32) g = g / 32 * 32;
+    long long items = 0;
+    for (int i = 0; i < t.n_jobs; ++i) {
+        t.jobs[i].vis_begin = items;
+        items += (long long)t.jobs[i].n_wtiles * ((t.jobs[i].n_vpl + g - 1) / g);
+    }
+    t.group = (int)g;
+    t.n_vis = (int)items;   // at most n_words
+    return true;
+}
+
 void batch_plan_destroy(BatchPlan *p) { delete p; }
 size_t batch_plan_partial_floats(const BatchPlan *p) { return p->partial_floats; }
 size_t batch_plan_order_bytes(const BatchPlan *p) {
@@ -235,10 +328,10 @@ int batch_plan_tables(const BatchPlan *p) { return (int)p->tables.size(); }
 int batch_plan_launches(const BatchPlan *p) {
     int n = 0;
     for (const OrderTable &o : p->orders) n += 2 + order_launches(o);
-    return n;
+    return n;   // one more per table launched in two passes
 }
 
-rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *work, int variant, int grid,
+rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *work, uint32_t *masks, int variant, int grid,
                              cudaStream_t st) {
     if (p->sorted_vpls > 0 && (!order || ((uintptr_t)order & 15u))) return RZK_ERR_INVALID;
     rzk_vpl *sorted = (rzk_vpl *)order;
@@ -258,11 +351,18 @@ rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *wor
     if (grid <= 0) grid = grid_for(variant);
     void *scratch = p->sorted_vpls > 0 ? (char *)order + up256(sizeof(rzk_vpl) * p->sorted_vpls) : nullptr;
     RZK_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int) * p->tables.size(), st));
+    if (masks && variant == 0 && p->vis_grid == 0) p->vis_grid = vis_grid();
+    const int vgrid = masks && variant == 0 ? p->vis_grid : 0;
     for (size_t k = 0; k < p->tables.size(); ++k) {
-        const JobTable &t = p->tables[k];
+        JobTable &t = p->tables[k];
         int *w = work + k;
         if (p->orders[k].total > 0) RZK_TRY(order_vpls(p->orders[k], scratch, sorted + p->order_base[k], st));
-        switch (variant) {
+        if (vgrid > 0 && plan_vis(t, vgrid)) {
+            batch_vis_kernel<4, 32, 7><<<vgrid, 128, 0, st>>>(t, w, masks);
+            RZK_CUDA_TRY(cudaGetLastError());
+            batch_shade_kernel<<<(unsigned)((32ll * t.n_items + kShadeBlock - 1) / kShadeBlock), kShadeBlock, 0, st>>>(
+                t, masks);
+        } else switch (variant) {
             case 0: batch_gather_kernel<4, 32, 7><<<grid, 128, 0, st>>>(t, w); break;
             case 1: batch_gather_kernel<4, 32, 6><<<grid, 128, 0, st>>>(t, w); break;
             case 2: batch_gather_kernel<2, 32, 1><<<grid, 64, 0, st>>>(t, w); break;
@@ -286,6 +386,7 @@ struct rzk_batch {
     float *d_partial = nullptr;
     void *d_order = nullptr;             // spatially ordered VPL copies and sort scratch
     int *d_work = nullptr;               // one work counter per table
+    uint32_t *d_masks = nullptr;         // visibility ballots of the two-pass tables (variant 0)
     int n_jobs = 0, variant = 0, grid = 0;
 };
 
@@ -300,6 +401,7 @@ rzk_status rzk_batch_destroy(rzk_batch *b) {
     if (b->d_partial) cudaFree(b->d_partial);
     if (b->d_order) cudaFree(b->d_order);
     if (b->d_work) cudaFree(b->d_work);
+    if (b->d_masks) cudaFree(b->d_masks);
     if (b->plan) batch_plan_destroy(b->plan);
     delete b;
     return RZK_OK;
@@ -328,6 +430,12 @@ rzk_status rzk_batch_create(rzk_context *ctx, const rzk_gather_job *jobs, int n_
     if ((e = cudaMalloc((void **)&bt->d_work, sizeof(int) * plan->tables.size())) != cudaSuccess) return fail(e);
     const size_t ob = batch_plan_order_bytes(plan);
     if (ob > 0 && (e = cudaMalloc(&bt->d_order, ob)) != cudaSuccess) return fail(e);
+    // without room for the ballots the batch runs in one pass
+    const size_t words = variant == 0 ? batch_plan_mask_words(plan) : 0;
+    if (words > 0 && cudaMalloc((void **)&bt->d_masks, sizeof(uint32_t) * words) != cudaSuccess) {
+        (void)cudaGetLastError();
+        bt->d_masks = nullptr;
+    }
     bt->grid = grid_for(variant);
     *out = bt;
     return RZK_OK;
@@ -335,7 +443,7 @@ rzk_status rzk_batch_create(rzk_context *ctx, const rzk_gather_job *jobs, int n_
 
 rzk_status rzk_batch_run(rzk_batch *b, void *stream) {
     if (!b) return RZK_ERR_INVALID;
-    return batch_plan_launch(b->plan, b->d_partial, b->d_order, b->d_work, b->variant, b->grid,
+    return batch_plan_launch(b->plan, b->d_partial, b->d_order, b->d_work, b->d_masks, b->variant, b->grid,
                              (cudaStream_t)stream);
 }
 

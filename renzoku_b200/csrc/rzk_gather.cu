@@ -552,17 +552,7 @@ __global__ void __launch_bounds__(kShadeBlock) gather_shade_kernel(DevScene s, c
         if (active) rm = load_material(s.mats + r.mat);
     }
     const int j0 = chunk * chunk_len, j1 = min(n_vpl, j0 + chunk_len);
-    const uint32_t *m = masks + (size_t)wt * n_vpl;
-    Rgb sum = crgb(0.0f, 0.0f, 0.0f);
-    for (int b = j0; b < j1; b += 32) {
-        const uint32_t word = b + lane < j1 ? __ldcs(m + b + lane) : 0u;
-        for (unsigned todo = __ballot_sync(kFull, word != 0u); todo; todo &= todo - 1u) {
-            const int v = __ffs(todo) - 1;
-            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
-            const rzk_vpl l = load_vpl(vpls + b + v);
-            sum = cadd(sum, pair_radiance(s, r, rm, l, pair_geo(r, l), mode, tau));
-        }
-    }
+    const Rgb sum = shade_marked(s, r, rm, vpls, j0, j1, masks + (size_t)wt * n_vpl + j0, mode, tau, lane);
     if (ri >= 0) {
         float *o = partial + 3 * ((size_t)chunk * n_recv + ri);
         __stcs(o, sum.r); __stcs(o + 1, sum.g); __stcs(o + 2, sum.b);

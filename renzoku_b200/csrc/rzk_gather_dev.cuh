@@ -210,7 +210,7 @@ __device__ __forceinline__ bool pair_clearly_zero(const RecvRegs &r, const rzk_v
     return pair_clearly_zero(r, l, vpl_power_finite(l), vpl_from_behind(l));
 }
 
-__device__ __forceinline__ Rgb pair_radiance(const DevScene &s, const RecvRegs &r, const rzk_material &rm,
+__device__ __forceinline__ Rgb pair_radiance(const GatherScene &s, const RecvRegs &r, const rzk_material &rm,
                                              const rzk_vpl &l, const PairGeo &pg, int mode, float tau) {
     Rgb sb = brdf_eval(rm, r.uvn, r.wo, pg.wi);
     Rgb lb;
@@ -232,7 +232,7 @@ __device__ __forceinline__ Rgb pair_radiance(const DevScene &s, const RecvRegs &
 // occludes the segment whichever way it was found, so a hit there is the traversal's
 // answer; the leaf of any triangle found becomes the lane's `cache`, the previous one its
 // `cache2`.
-__device__ __forceinline__ bool packet_visible_near(const DevScene &s, const Ray &ray, float tmax, bool act,
+__device__ __forceinline__ bool packet_visible_near(const GatherScene &s, const Ray &ray, float tmax, bool act,
                                                     int *stk, int &cache, int &cache2) {
     if (s.n_nodes == 0) return act;
     const float4 lo = __ldg(s.trav + 2), hi = __ldg(s.trav + 3);
@@ -394,7 +394,7 @@ __host__ __device__ __forceinline__ long long warp_tiles(long long n_recv, int i
 // word), and the item then returns false.  The tile shape changes which receivers share a
 // packet, never a receiver's sum.
 template <int TILE, int TW = 8, class Sink>
-__device__ __forceinline__ bool gather_item(const DevScene &s, const rzk_receiver *recv, int n_recv, int img_w,
+__device__ __forceinline__ bool gather_item(const GatherScene &s, const rzk_receiver *recv, int n_recv, int img_w,
                                             const rzk_vpl *vpls, int n_vpl, int chunk, int wt, int chunk_len,
                                             int mode, float tau, WarpStage<TILE> &ws, int lane, Sink &&sink) {
     const int ri = lane_receiver<TW>(wt, lane, n_recv, img_w);
@@ -495,7 +495,7 @@ struct PlaneSink {
 // is unoccluded - exactly the pairs gather_item adds.  Returns false if a bounded wait gave
 // up (reported in the error word).
 template <int TILE>
-__device__ __forceinline__ bool visibility_item(const DevScene &s, const rzk_receiver *recv, int n_recv, int img_w,
+__device__ __forceinline__ bool visibility_item(const GatherScene &s, const rzk_receiver *recv, int n_recv, int img_w,
                                                 const rzk_vpl *vpls, int j0, int j1, int wt, WarpStage<TILE> &ws,
                                                 int lane, uint32_t *masks) {
     const int ri = lane_receiver(wt, lane, n_recv, img_w);
@@ -561,12 +561,30 @@ __device__ __forceinline__ bool visibility_item(const DevScene &s, const rzk_rec
     return true;
 }
 
+// Summing half for one warp: each lane's sum, in VPL order, of its receiver's terms with the VPLs
+// of [j0, j1) that `masks` (first word: VPL j0's, from visibility_item) marks.
+__device__ __forceinline__ Rgb shade_marked(const GatherScene &s, const RecvRegs &r, const rzk_material &rm,
+                                            const rzk_vpl *vpls, int j0, int j1, const uint32_t *masks, int mode,
+                                            float tau, int lane) {
+    Rgb sum = crgb(0.0f, 0.0f, 0.0f);
+    for (int b = j0; b < j1; b += 32) {
+        const uint32_t word = b + lane < j1 ? __ldcs(masks + (b - j0) + lane) : 0u;
+        for (unsigned todo = __ballot_sync(kFull, word != 0u); todo; todo &= todo - 1u) {
+            const int v = __ffs(todo) - 1;
+            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
+            const rzk_vpl l = load_vpl(vpls + b + v);
+            sum = cadd(sum, pair_radiance(s, r, rm, l, pair_geo(r, l), mode, tau));
+        }
+    }
+    return sum;
+}
+
 // Summing half with one order of additions per sum but the terms formed in parallel: the warps
 // of a block (at least three) take the VPLs of [j0, j1) in turn, 32 VPLs at a time, and leave the
 // terms in `terms`; then thread t < 96 adds channel t / 32 of receiver t % 32 in VPL order.
 // Returns that thread's sum.  `masks` as from visibility_item, its first word VPL j0's.
 template <int WARPS>
-__device__ __forceinline__ float shade_chunk(const DevScene &s, const RecvRegs &r, bool active, const rzk_vpl *vpls,
+__device__ __forceinline__ float shade_chunk(const GatherScene &s, const RecvRegs &r, bool active, const rzk_vpl *vpls,
                                              int j0, int j1, const uint32_t *masks, int mode, float tau,
                                              float (*terms)[3][32]) {
     static_assert(WARPS >= 3, "a warp per channel");
@@ -606,7 +624,7 @@ __device__ __forceinline__ float shade_chunk(const DevScene &s, const RecvRegs &
 // WEIGHTED: VPL j's radiance is multiplied by weights[j] before it is added (a cluster
 // representative standing for its cluster).  Writes partial[3 * ri ...].
 template <bool WEIGHTED>
-__device__ __forceinline__ void shade_item(const DevScene &s, const rzk_receiver *recv, int n_recv, int img_w,
+__device__ __forceinline__ void shade_item(const GatherScene &s, const rzk_receiver *recv, int n_recv, int img_w,
                                            const rzk_vpl *vpls, int n_vpl, const uint32_t *masks, int wt, int mode,
                                            float tau, float *partial, int lane, const float *weights) {
     const int ri = lane_receiver(wt, lane, n_recv, img_w);

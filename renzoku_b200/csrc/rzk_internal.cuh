@@ -65,26 +65,31 @@ struct DevLight {
     int kind, flags, n_tris;
 };
 
-// Everything a kernel needs to trace and shade in one scene (passed by value).
-struct DevScene {
-    const float4 *nodes;      // 2 x float4 per slot, slot = BFS node index + 1
+// What the gather kernels need of a scene.
+struct GatherScene {
+    const float4 *trav;       // any-hit tree, same packing as nodes (rzk_sah.cu; = nodes without it)
     const float4 *tri_isect;  // 3 x float4 per sorted triangle (see tri_hit)
+    const rzk_material *mats;
+    uint32_t *err;            // device error word (context-owned)
+    unsigned long long *rays; // shadow rays traced by the gather kernels (context-owned counter)
+    int n_nodes;
+    float tmin;
+};
+
+// Everything a kernel needs to trace and shade in one scene (passed by value).
+struct DevScene : GatherScene {
+    const float4 *nodes;      // 2 x float4 per slot, slot = BFS node index + 1
     const float4 *tri_shade;  // 2 x float4 per sorted triangle: {n, surf}, {u, -}
     const float4 *wide;       // 8 x float4 per 4-wide traversal node (see rzk_bvh.cu K6)
-    const float4 *trav;       // any-hit tree, same packing as nodes (rzk_sah.cu; = nodes without it)
     const float4 *ctrav;      // closest-hit tree: trav with inflated boxes (rzk_sah.cu), or null
     const float *verts;       // 9 per triangle in input order
     const int *perm;          // sorted triangle slot -> input triangle
     const int4 *surf;         // per surface {mat, flags, light, -}
-    const rzk_material *mats;
     const DevLight *lights;
     const float *light_pdf;
     const float *light_cdf;
-    int n_tris, n_nodes, n_mats, n_lights;
-    float tmin;
+    int n_tris, n_mats, n_lights;
     float cguard[4];          // origins ctrav covers: centre, squared radius
-    uint32_t *err;            // device error word (context-owned)
-    unsigned long long *rays; // shadow rays traced by the gather kernels (context-owned counter)
 };
 
 struct Scene;
@@ -244,6 +249,9 @@ size_t batch_plan_partial_floats(const BatchPlan *p);
 size_t batch_plan_order_bytes(const BatchPlan *p);
 int batch_plan_tables(const BatchPlan *p);
 int batch_plan_launches(const BatchPlan *p);   // kernels one batch_plan_launch launches
-rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *work, int variant, int grid,
+// masks: null, or batch_plan_mask_words words, with which the tables that a two-pass launch
+// suits run in two passes (as rzk_gather does; variant 0 only, the same images).
+size_t batch_plan_mask_words(const BatchPlan *p);
+rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *work, uint32_t *masks, int variant, int grid,
                              cudaStream_t st);
 }  // namespace rzk

@@ -189,7 +189,7 @@ void launch_group(rzk_server *s, Group *g) {
                 cudaMallocAsync((void **)&work, sizeof(int) * rzk::batch_plan_tables(plan), st) != cudaSuccess)
                 r = RZK_ERR_NOMEM;
         }
-        if (r == RZK_OK) r = rzk::batch_plan_launch(plan, partial, order, work, 0, 0, st);
+        if (r == RZK_OK) r = rzk::batch_plan_launch(plan, partial, order, work, nullptr, 0, 0, st);
         if (r == RZK_OK) g->launches += rzk::batch_plan_launches(plan);
         if (partial) cudaFreeAsync(partial, st);
         if (order) cudaFreeAsync(order, st);

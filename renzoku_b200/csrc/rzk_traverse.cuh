@@ -43,7 +43,7 @@ struct TraceStats {
     __device__ __forceinline__ void reset() { inner = 0; leaf = 0; }
 };
 
-__device__ __forceinline__ void load_tri(const DevScene &s, int slot, float4 &a, float4 &b, float4 &c) {
+__device__ __forceinline__ void load_tri(const GatherScene &s, int slot, float4 &a, float4 &b, float4 &c) {
     const float4 *p = s.tri_isect + 3 * slot;
     a = __ldg(p); b = __ldg(p + 1); c = __ldg(p + 2);
 }
