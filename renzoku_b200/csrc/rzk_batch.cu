@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_vis_kernel(const __gri
                                                                      uint32_t *masks) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_gather_kernel(const __
                                                                         int *work) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
@@ -299,7 +299,7 @@ static int vis_grid() {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_vis_kernel<4, 32, 7>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_vis_kernel<4, 16, 7>, 128, 0);
     return std::max(1, sms * std::max(1, per_sm));
 }
 
@@ -358,7 +358,7 @@ rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *wor
         int *w = work + k;
         if (p->orders[k].total > 0) RZK_TRY(order_vpls(p->orders[k], scratch, sorted + p->order_base[k], st));
         if (vgrid > 0 && plan_vis(t, vgrid)) {
-            batch_vis_kernel<4, 32, 7><<<vgrid, 128, 0, st>>>(t, w, masks);
+            batch_vis_kernel<4, 16, 7><<<vgrid, 128, 0, st>>>(t, w, masks);
             RZK_CUDA_TRY(cudaGetLastError());
             batch_shade_kernel<<<(unsigned)((32ll * t.n_items + kShadeBlock - 1) / kShadeBlock), kShadeBlock, 0, st>>>(
                 t, masks);

@@ -575,6 +575,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
         }
         RZK_TRY(build_closest_tree(s, st));
     }
+    RZK_TRY(build_wide_tree(s, st));
     return RZK_OK;
 }
 

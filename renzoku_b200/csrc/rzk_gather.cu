@@ -166,7 +166,7 @@ __device__ __forceinline__ Rgb shade_cull(const DevScene &s, const RecvRegs &r, 
 }
 
 // Packet any-hit for the lanes in `act`; returns the lanes that stay unoccluded.
-__device__ __forceinline__ bool packet_visible(const DevScene &s, const Ray &ray, float tmax, bool act,
+__device__ __forceinline__ bool packet_visible_binary(const DevScene &s, const Ray &ray, float tmax, bool act,
                                                int *stk) {
     if (s.n_nodes == 0) return act;
     const float4 lo = __ldg(s.nodes + 2), hi = __ldg(s.nodes + 3);
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(WARPS * 32) gather_packet_kernel(DevScene s, c
             V3 q = ld3(l.p);
             Ray ray = make_ray(r.p, sub(q, r.p));
             float tmax = len(sub(q, r.p)) - s.tmin;
-            bool vis = WIDE ? packet_visible_wide(s, ray, tmax, act, stk) : packet_visible(s, ray, tmax, act, stk);
+            bool vis = WIDE ? packet_visible_wide(s, ray, tmax, act, stk) : packet_visible_binary(s, ray, tmax, act, stk);
             if (vis) sum = cadd(sum, L);
         }
         __syncwarp();
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(WARPS * 32) gather_packet_kernel(DevScene s, c
 // while another still holds long work (the tail of a fixed grid cost about 40% of the
 // issue slots).  Per VPL the lanes first apply only the BRDFs' early-outs (the exact zero
 // tests of lambertian.cc:63-66, phong.cc:74-77, ward.cc:104-109); the surviving lanes
-// trace their shadow rays as a packet, nearer child first by majority; the full BRDF
+// trace their shadow rays as a packet (packet_visible); the full BRDF
 // values and the clamp are evaluated only for the lanes that stay visible (about 80% of
 // traced shadow rays are occluded on the scaled scene).  Each lane adds its terms in VPL
 // order; the chunk sums are added in chunk order by reduce_chunks_kernel after the launch
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_persistent_kernel(
     ChunkRing ring, float *out) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_vis_kernel(DevScene s
                                                                       uint32_t *masks) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
@@ -914,7 +914,7 @@ struct GatherVariant {
     int kind, warps_or_block, tile, tw;
 };
 static const GatherVariant kVariants[] = {
-    {3, 4, 32, 8}, {3, 2, 32, 8}, {3, 4, 32, 8}, {3, 4, 32, 8}, {1, 4, 32, 8}, {1, 2, 32, 8}, {2, 4, 32, 8},
+    {3, 4, 16, 8}, {3, 2, 32, 8}, {3, 4, 32, 8}, {3, 4, 32, 8}, {1, 4, 32, 8}, {1, 2, 32, 8}, {2, 4, 32, 8},
     {0, 128, 64, 8}, {3, 4, 32, 4}, {3, 4, 32, 16}, {3, 4, 32, 32}};
 
 int gather_variant_count() { return (int)(sizeof(kVariants) / sizeof(kVariants[0])); }
@@ -977,7 +977,7 @@ static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, 
         int dev = 0, sms = 0, per_sm = 0;
         RZK_CUDA_TRY(cudaGetDevice(&dev));
         RZK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 32, 7>, 128, 0));
+        RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 16, 7>, 128, 0));
         ctx->vis_grid = std::max(1, sms * std::max(1, per_sm));
     }
     group = (int)std::min<long long>(kMaxGroup, std::max<long long>(1, wtiles * n_vpl / (kItems * 4 * ctx->vis_grid)));
@@ -1019,7 +1019,7 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
         const int n_groups = (n_vpl + group - 1) / group;
         RZK_CUDA_TRY(cudaMemsetAsync(ctx->d_work, 0, sizeof(int), st));
         const long long blocks = std::min<long long>(ctx->vis_grid, (wtiles * n_groups + 3) / 4);
-        gather_vis_kernel<4, 32, 7><<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, group, n_groups,
+        gather_vis_kernel<4, 16, 7><<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, group, n_groups,
                                                                       (int)wtiles, ctx->d_work, masks);
         RZK_CUDA_TRY(cudaGetLastError());
         const long long items = wtiles * n_chunks;
@@ -1036,7 +1036,7 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
         switch (variant) {
             case 2: gather_persistent_kernel<4, 32, 1><<<persistent_grid<4, 32, 1>(ctx, 2), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
             case 1: gather_persistent_kernel<2, 32, 1><<<persistent_grid<2, 32, 1>(ctx, 1), 64, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
-            case 0: gather_persistent_kernel<4, 32, 7><<<persistent_grid<4, 32, 7>(ctx, 0), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
+            case 0: gather_persistent_kernel<4, 16, 7><<<persistent_grid<4, 16, 7>(ctx, 0), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
             case 8: gather_persistent_kernel<4, 32, 5, 4><<<persistent_grid<4, 32, 5, 4>(ctx, 8), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
             case 9: gather_persistent_kernel<4, 32, 5, 16><<<persistent_grid<4, 32, 5, 16>(ctx, 9), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
             case 10: gather_persistent_kernel<4, 32, 5, 32><<<persistent_grid<4, 32, 5, 32>(ctx, 10), 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, wt, ctx->d_work, mode, tau, part, scale, nr, out); break;
@@ -1097,7 +1097,7 @@ rzk_status launch_mean(rzk_context *ctx, const DevScene &s, const rzk_receiver *
     return RZK_OK;
 }
 
-// The persistent gather (4 warps, 32-VPL tiles, 7 CTAs per SM, 8 x 4 warp tiles) on
+// The persistent gather (4 warps, 16-VPL tiles, 7 CTAs per SM, 8 x 4 warp tiles) on
 // caller-provided scratch: a chunk ring in `ring_mem` with as many tile slots as its
 // `ring_mem_bytes` hold (up to kRingSlots; RZK_ERR_CAPACITY when not one fits) and the work
 // counter `work`, both zeroed on `st` first.  n_chunks as resolved by the caller (chunk
@@ -1131,14 +1131,14 @@ rzk_status launch_gather_scratch(const DevScene &s, const rzk_receiver *recv, in
         int sms = 0, per_sm = 0;
         g.err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (g.err == cudaSuccess)
-            g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_persistent_kernel<4, 32, 7, 8, true>,
+            g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_persistent_kernel<4, 16, 7, 8, true>,
                                                                   128, 0);
         g.blocks = std::max(1, sms * std::max(1, per_sm));
     });
     RZK_CUDA_TRY(g.err);
     RZK_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int), st));
     RZK_CUDA_TRY(cudaMemsetAsync(ring_mem, 0, ring_counter_bytes(slots), st));
-    gather_persistent_kernel<4, 32, 7, 8, true><<<g.blocks, 128, 0, st>>>(
+    gather_persistent_kernel<4, 16, 7, 8, true><<<g.blocks, 128, 0, st>>>(
         s, recv, n_recv, img_w, vpls, n_vpl, chunk_len, n_chunks, (int)wtiles, work, mode, tau, nullptr, scale,
         ring_at(ring_mem, slots), out);
     RZK_CUDA_TRY(cudaGetLastError());

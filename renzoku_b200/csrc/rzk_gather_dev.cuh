@@ -224,137 +224,202 @@ __device__ __forceinline__ Rgb pair_radiance(const GatherScene &s, const RecvReg
     return radiance_terms(pg.power, sb, lb, pg.G, mode, tau);
 }
 
-// Packet any-hit, nearer child first by lane majority.  Returns whether this lane's
-// segment is unoccluded (lanes with act == false return false).
-// `cache` and `cache2` (per lane) name the any-hit-tree leaves whose triangles last
-// occluded this lane's receiver (most recent first), or -1.  They are tried first, then the
-// leaves cached by five neighbouring lanes: a triangle whose own box and triangle tests pass
-// occludes the segment whichever way it was found, so a hit there is the traversal's
-// answer; the leaf of any triangle found becomes the lane's `cache`, the previous one its
-// `cache2`.
-__device__ __forceinline__ bool packet_visible_near(const GatherScene &s, const Ray &ray, float tmax, bool act,
-                                                    int *stk, int &cache, int &cache2) {
-    if (s.n_nodes == 0) return act;
-    const float4 lo = __ldg(s.trav + 2), hi = __ldg(s.trav + 3);
-    float t_root = 0.0f;
-    bool alive = act && box_hit_fast(lo, hi, ray, s.tmin, tmax, t_root);
-    if (!__any_sync(kFull, alive)) return act;
-    const int a = __float_as_int(lo.w);
-    if (a < 0) {
-        if (alive) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - a, ta, tb, tc);
-            if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) return false;
-        }
-        return act;
-    }
-    bool occluded = false;
-    if (alive && cache >= 0) {
-        const float4 *pc = s.trav + 2 * (cache + 1);
-        const float4 c0 = __ldg(pc), c1 = __ldg(pc + 1);
-        float tc0 = 0.0f;
-        if (box_hit_fast(c0, c1, ray, s.tmin, tmax, tc0)) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - __float_as_int(c0.w), ta, tb, tc);
-            if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) occluded = true;
-        }
-    }
-    if (alive && !occluded && cache2 >= 0 && cache2 != cache) {   // the one before it
-        const float4 *pc = s.trav + 2 * (cache2 + 1);
-        const float4 c0 = __ldg(pc), c1 = __ldg(pc + 1);
-        float tc0 = 0.0f;
-        if (box_hit_fast(c0, c1, ray, s.tmin, tmax, tc0)) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - __float_as_int(c0.w), ta, tb, tc);
-            if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) {
-                occluded = true;
-                const int t = cache;
-                cache = cache2;
-                cache2 = t;
-            }
-        }
-    }
-    // Then the leaves cached by the lanes at xor distances 1, 8, 2, 16 and 4: in an 8 x 4
-    // pixel tile those are the neighbouring pixels, whose shadow rays toward the same VPL
-    // run almost parallel and are often blocked by the same triangle.  The same rule
-    // applies (own box and triangle tests), so the answer is still exact; a lane blocked by
-    // a neighbour's leaf adopts it.  Every lane takes part in each shuffle.
-    constexpr int kNeighbours[5] = {1, 8, 2, 16, 4};
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-        const int other = __shfl_xor_sync(kFull, cache, kNeighbours[q]);
-        if (alive && !occluded && other >= 0 && other != cache) {
-            const float4 *pc = s.trav + 2 * (other + 1);
-            const float4 c0 = __ldg(pc), c1 = __ldg(pc + 1);
-            float tc0 = 0.0f;
-            if (box_hit_fast(c0, c1, ray, s.tmin, tmax, tc0)) {
-                float4 ta, tb, tc;
-                load_tri(s, -1 - __float_as_int(c0.w), ta, tb, tc);
-                if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) {
-                    occluded = true;
-                    cache2 = cache;
-                    cache = other;
-                }
-            }
-        }
-    }
-    // every lane takes part in the vote (the cache tests above are per lane)
-    alive = alive && !occluded;
-    if (!__any_sync(kFull, alive)) return act && !occluded;
-    // lanes whose root test failed cannot reach any triangle below it: they stay visible.
-    // The warp descends straight into the child it visits next (the nearer one where both
-    // are entered) and pushes only the other: the visit order of a push-both stack, without
-    // a shared-memory store and load on the step's dependency chain.
-    int top = -1;
-    int c = a;
-    bool overflow = false;
-    for (;;) {
-        const float4 *pn = s.trav + 2 * (c + 1);
-        const float4 l0 = __ldg(pn), l1 = __ldg(pn + 1), r0 = __ldg(pn + 2), r1 = __ldg(pn + 3);
-        const int al = __float_as_int(l0.w), ar = __float_as_int(r0.w);
-        float tl = 0.0f, tr = 0.0f;
-        bool hl = alive && box_hit_fast(l0, l1, ray, s.tmin, tmax, tl);
-        bool hr = alive && box_hit_fast(r0, r1, ray, s.tmin, tmax, tr);
-        if (al < 0 && hl && !occluded) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - al, ta, tb, tc);
-            if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) {
-                occluded = true;
-                if (cache != c) { cache2 = cache; cache = c; }
-            }
-        }
-        if (ar < 0 && hr && !occluded) {
-            float4 ta, tb, tc;
-            load_tri(s, -1 - ar, ta, tb, tc);
-            if (tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) {
-                occluded = true;
-                if (cache != c + 1) { cache2 = cache; cache = c + 1; }
-            }
-        }
-        alive = alive && !occluded;
-        const bool pl = al >= 0 && __any_sync(kFull, hl && alive);
-        const bool pr = ar >= 0 && __any_sync(kFull, hr && alive);
-        if (!__any_sync(kFull, alive)) break;
-        if (pl && pr) {
-            // visit the child most live lanes enter first; the other waits on the stack
-            unsigned left_first = __ballot_sync(kFull, alive && hl && hr && tl <= tr);
-            unsigned right_first = __ballot_sync(kFull, alive && hl && hr && tr < tl);
-            const int first = __popc(left_first) >= __popc(right_first) ? al : ar;
-            if (top < STACK_CAP - 1) stk[++top] = first == al ? ar : al; else overflow = true;
-            c = first;
-        } else if (pl) {
-            c = al;
-        } else if (pr) {
-            c = ar;
-        } else {
-            if (top < 0) break;
-            c = stk[top--];
-        }
-    }
-    if (overflow && s.err) atomicOr(s.err, ERR_STACK);
-    return act && !occluded;
+__device__ __forceinline__ float warp_min_f(float x) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f(float x) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
 }
 
+// The shaft of a warp's shadow segments: all end at the VPL q, so a point of any of them is
+// q + s (p - q) with s in [0, 1] and, per axis, p - q within [umin, umax] over the live lanes.
+// A box [lo, hi] meets the shaft only if some s lies, on every axis, between the least and the
+// largest s for which an s u of that interval reaches into [lo - q, hi - q].  The test below
+// passes every box that box_hit_fast passes for one of the segments: a float slab test accepts
+// points within 3 u (|plane| + |origin|) of the box, the float direction is within 4 u of
+// (q - p) / |q - p|, and a direction component below 1e-6 is replaced by it (2e-6 of the
+// distance); the planes are moved out by 8e-6 of the coordinates' size, the interval of u by as
+// much, and the quotients by 2e-6 of themselves.  Comparisons that a NaN spoils pass.
+struct Shaft {
+    float qa[3], qb[3];   // q plus and minus the margin
+    float n1[3], n2[3];   // entry: max((lo - qa) n1, (hi - qb) n2)
+    float f[3], g[3];     // exit:  ((hi - qb), or where u < 0 (lo - qa)) f + g
+    bool neg[3];
+    __device__ __forceinline__ void set(V3 q, V3 p, bool live) {
+        const float qv[3] = {q.x, q.y, q.z}, pv[3] = {p.x, p.y, p.z};
+        float lo[3], hi[3], size = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float u = pv[a] - qv[a];
+            lo[a] = warp_min_f(live ? u : INFINITY);
+            hi[a] = warp_max_f(live ? u : -INFINITY);
+            size = fmaxf(size, fabsf(qv[a]) + fmaxf(fabsf(lo[a]), fabsf(hi[a])));
+        }
+        const float eps = 8e-6f * size;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            qa[a] = qv[a] + eps;
+            qb[a] = qv[a] - eps;
+            const float u0 = lo[a] - eps, u1 = hi[a] + eps;
+            const float r0 = __fdividef(1.0f, u0), r1 = __fdividef(1.0f, u1);
+            const bool pos = u0 > 0.0f;
+            neg[a] = u1 < 0.0f;
+            n1[a] = neg[a] ? 0.0f : 0.999998f * r1;
+            n2[a] = pos ? 0.0f : 0.999998f * r0;
+            f[a] = 1.000002f * (pos ? r0 : neg[a] ? r1 : 0.0f);
+            g[a] = pos || neg[a] ? 0.0f : 1e30f;
+        }
+    }
+    __device__ __forceinline__ bool meets(float4 lo, float4 hi) const {
+        const float l[3] = {lo.x - qa[0], lo.y - qa[1], lo.z - qa[2]};
+        const float h[3] = {hi.x - qb[0], hi.y - qb[1], hi.z - qb[2]};
+        float near = -2e-6f, far = 1.000002f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            near = fmaxf(near, fmaxf(l[a] * n1[a], h[a] * n2[a]));
+            far = fminf(far, __fmaf_rn(neg[a] ? l[a] : h[a], f[a], g[a]));
+        }
+        return !(near > far);
+    }
+};
+
+// Packet any-hit over the 8-wide any-hit tree.  Returns whether this lane's segment is
+// unoccluded (lanes with act == false return false).
+//
+// `cache` and `cache2` (per lane) name the entries of the tree whose triangles last
+// occluded this lane's receiver (most recent first), or -1.  They are tried first, then the
+// entries cached by five neighbouring lanes: a triangle whose own box and triangle tests pass
+// occludes the segment whichever way it was found, so a hit there is the traversal's
+// answer; the entry of any triangle found becomes the lane's `cache`, the previous one its
+// `cache2`.
+//
+// The walk tests nodes against the whole packet, not rays against nodes: a lane holds one child
+// of one of up to four 8-wide nodes and tests its box against the packet's shaft, so a step
+// covers 32 boxes; every leaf whose box meets the shaft is then tested by each live lane with its
+// own ray (box, then triangle).  The answer is exact: a triangle is looked at whenever its own
+// box passes for some lane, because the shaft test passes wherever box_hit_fast does, and it
+// occludes a lane only by that lane's own tests.  A packet whose rays are far apart for the
+// triangles' size (a 192-pixel image: 81 leaves in the shaft, 6 of them entered) refines a step's
+// boxes by the rays themselves, each lane its box against every live ray.
+//
+// Bound by the issue rate.  One ray per lane and two boxes a step took about 95 instructions for
+// 2 boxes, 40 steps a packet; this takes about 80 for 32, 7 to 12 steps.  512 x 512 x 32,768 VPLs,
+// 300k triangles 103 -> 61 ms; ten requests of up to 192 x 192 x 3,000, 10k to 30k triangles
+// 37.5 -> 23.7 (64 without the refinement; its limit at 4 m > live + 8: 25.0, m > live: 33.2,
+// 2 m > live + 12: 24.3); LightSlice's tracing 11.6 -> 5.4; 36 triangles 8.1 -> 7.5 (B200, with
+// VPL tiles of 16 instead of 32, which leave L1 124 KB instead of 28: 103 -> 73 ms with 32).
+constexpr int kWideFan = 8;
+constexpr int kWideMulti = 64;    // most pending nodes with which four are taken at once
+// from at most kWideMulti + 28 pending, one node at a time adds at most 7 a level; 21 levels of a
+// 62-deep binary tree taken three at a time
+constexpr int kWideStack = kWideMulti + 28 + 7 * 21 + 1;
+constexpr int kPacketInts = kWideStack + 64;   // a packet's shared memory: pending nodes, listed leaves
+
+__device__ __forceinline__ bool entry_occludes(const GatherScene &s, int entry, const Ray &ray, float tmax) {
+    const float4 *p = s.wide8 + 2 * (size_t)entry;
+    const float4 lo = __ldg(p), hi = __ldg(p + 1);
+    float t = 0.0f;
+    if (!box_hit_fast(lo, hi, ray, s.tmin, tmax, t)) return false;
+    float4 ta, tb, tc;
+    load_tri(s, -1 - __float_as_int(lo.w), ta, tb, tc);
+    return tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr);
+}
+
+__device__ __forceinline__ bool packet_visible(const GatherScene &s, V3 p, V3 q, const Ray &ray, float tmax, bool act,
+                                               int *stk, int &cache, int &cache2) {
+    if (s.n_nodes == 0) return act;
+    const int lane = threadIdx.x & 31;
+    bool alive = act;
+    // The lane's own two entries, then those cached by the lanes at xor distances 1, 8, 2, 16 and
+    // 4: in an 8 x 4 pixel tile those are the neighbouring pixels, whose shadow rays toward the
+    // same VPL run almost parallel and are often blocked by the same triangle.  The same rule
+    // applies (own box and triangle tests), so the answer is still exact; a lane blocked by
+    // a neighbour's entry adopts it.  Every lane takes part in each shuffle.  One copy of the
+    // tests: unrolled, the kernels outgrow the instruction cache.
+    constexpr unsigned long long kDistance = 0x041002080100ull << 8;   // one byte a round: 0, 0, 1, 8, 2, 16, 4
+#pragma unroll 1
+    for (int k = 0; k < 7; ++k) {
+        const int other = __shfl_xor_sync(kFull, k == 1 ? cache2 : cache, (int)((kDistance >> (8 * k)) & 31u));
+        if (alive && other >= 0 && (k == 0 || other != cache) && entry_occludes(s, other, ray, tmax)) {
+            alive = false;
+            if (k > 0) {
+                cache2 = cache;
+                cache = other;
+            }
+        }
+        if (!__any_sync(kFull, alive)) return false;
+    }
+
+    Shaft sh;
+    sh.set(q, p, alive);
+    int n = 1;
+    if (lane == 0) stk[0] = 0;
+    __syncwarp();
+    const unsigned below = (1u << lane) - 1u;
+    do {
+        const int take = n <= kWideMulti ? min(n, 4) : 1;
+        n -= take;
+        bool meets = false;
+        int entry = 0, code = 0;
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        if ((lane >> 3) < take) {
+            entry = stk[n + (lane >> 3)] * kWideFan + (lane & 7);
+            const float4 *e = s.wide8 + 2 * (size_t)entry;
+            lo = __ldg(e);
+            hi = __ldg(e + 1);
+            code = __float_as_int(lo.w);
+            meets = code != kWideEmpty && sh.meets(lo, hi);
+        }
+        // a wide packet's shaft holds many boxes that no ray enters: where they are many against
+        // the live lanes, each lane tests its box with every live ray
+        unsigned live = __ballot_sync(kFull, alive);
+        if (2 * __popc(__ballot_sync(kFull, meets)) > __popc(live) + 8) {
+            bool entered = false;
+            for (; live; live &= live - 1u) {
+                const int k = __ffs(live) - 1;
+                Ray other;
+                other.inv_d = mk(__shfl_sync(kFull, ray.inv_d.x, k), __shfl_sync(kFull, ray.inv_d.y, k),
+                                 __shfl_sync(kFull, ray.inv_d.z, k));
+                other.org_inv_d = mk(__shfl_sync(kFull, ray.org_inv_d.x, k), __shfl_sync(kFull, ray.org_inv_d.y, k),
+                                     __shfl_sync(kFull, ray.org_inv_d.z, k));
+                const float far = __shfl_sync(kFull, tmax, k);
+                float t = 0.0f;
+                entered |= box_hit_fast(lo, hi, other, s.tmin, far, t);
+            }
+            meets = meets && entered;
+        }
+        const unsigned inner = __ballot_sync(kFull, meets && code >= 0);
+        if (inner) {
+            if (n + __popc(inner) > kWideStack) {   // not met: a tree deeper than the stack covers
+                if (lane == 0 && s.err) atomicOr(s.err, ERR_STACK);
+                break;
+            }
+            if (meets && code >= 0) stk[n + __popc(inner & below)] = code;
+            n += __popc(inner);
+            __syncwarp();
+        }
+        for (unsigned leaf = __ballot_sync(kFull, meets && code < 0); leaf; leaf &= leaf - 1u) {
+            const int e = __shfl_sync(kFull, entry, __ffs(leaf) - 1);
+            const float4 *pe = s.wide8 + 2 * (size_t)e;
+            const float4 lo = __ldg(pe), hi = __ldg(pe + 1);
+            float t = 0.0f;
+            const bool in = alive && box_hit_fast(lo, hi, ray, s.tmin, tmax, t);
+            if (!__any_sync(kFull, in)) continue;
+            float4 ta, tb, tc;
+            load_tri(s, -1 - __float_as_int(lo.w), ta, tb, tc);
+            if (in && tri_hit<false>(ta, tb, tc, ray, s.tmin, tmax, nullptr, nullptr, nullptr)) {
+                alive = false;
+                if (cache != e) { cache2 = cache; cache = e; }
+            }
+            if (!__any_sync(kFull, alive)) return false;
+        }
+    } while (n > 0);
+    return alive;
+}
 
 // Per-warp staging state of the persistent gathers: the warp's two VPL tiles, their
 // barriers (with the number of completed phases of each) and its packet stack.
@@ -457,7 +522,7 @@ __device__ __forceinline__ bool gather_item(const GatherScene &s, const rzk_rece
             n_rays += (unsigned)__popc(am);
             Ray ray = make_ray(r.p, sub(pg.q, r.p));
             float tmax = len(sub(pg.q, r.p)) - s.tmin;
-            if (packet_visible_near(s, ray, tmax, act, ws.stk, occ_cache, occ_cache2)) {
+            if (packet_visible(s, r.p, ld3(l.p), ray, tmax, act, ws.stk, occ_cache, occ_cache2)) {
                 // the pair's geometry (recomputed: the same operations on the same values),
                 // the material and the receiver's tangent basis are read or formed again here
                 // rather than held in registers through the traversal
@@ -551,7 +616,7 @@ __device__ __forceinline__ bool visibility_item(const GatherScene &s, const rzk_
             Ray ray = make_ray(r.p, sub(pg.q, r.p));
             float tmax = len(sub(pg.q, r.p)) - s.tmin;
             const unsigned vis =
-                __ballot_sync(kFull, packet_visible_near(s, ray, tmax, act, ws.stk, occ_cache, occ_cache2));
+                __ballot_sync(kFull, packet_visible(s, r.p, ld3(l.p), ray, tmax, act, ws.stk, occ_cache, occ_cache2));
             if (lane == v) word = vis;
         }
         if (lane < cnt) masks[k * TILE + lane] = word;

@@ -67,6 +67,7 @@ struct DevLight {
 
 // What the gather kernels need of a scene.
 struct GatherScene {
+    const float4 *wide8;      // 8-wide any-hit tree: 16 x float4 per node (rzk_sah.cu)
     const float4 *trav;       // any-hit tree, same packing as nodes (rzk_sah.cu; = nodes without it)
     const float4 *tri_isect;  // 3 x float4 per sorted triangle (see tri_hit)
     const rzk_material *mats;
@@ -143,6 +144,8 @@ struct rzk_scene {
     float4 *d_wide = nullptr;
     int n_wide = 0, n_wide_cap = 0;
     float4 *d_trav = nullptr;    // SAH any-hit tree (rzk_sah.cu)
+    float4 *d_wide8 = nullptr;   // 8-wide any-hit tree of the packet gathers (rzk_sah.cu), not saved
+    int n_wide8 = 0;             // nodes it has room for
     float4 *d_ctrav = nullptr;   // closest-hit tree (rzk_sah.cu), not saved: made from d_trav
     size_t ctrav_bytes = 0;
     float cguard[4] = {0, 0, 0, -1};
@@ -163,6 +166,7 @@ struct rzk_scene {
         rzk::DevScene s;
         s.nodes = d_nodes; s.tri_isect = d_tri_isect; s.tri_shade = d_tri_shade; s.wide = d_wide;
         s.trav = d_trav ? d_trav : d_nodes;
+        s.wide8 = d_wide8;
         s.ctrav = d_ctrav;
         for (int i = 0; i < 4; ++i) s.cguard[i] = cguard[i];
         s.verts = d_v;
@@ -181,6 +185,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st);
 // rzk_sah.cu
 rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st);
 rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st);
+rzk_status build_wide_tree(rzk_scene *s, cudaStream_t st);
 // utilities (rzk_bvh.cu)
 rzk_status exclusive_scan_i32(const int *d_in, int *d_out, int n, int *d_total, void *d_tmp,
                               size_t tmp_bytes, cudaStream_t st);

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) cluster_vis_kernel(DevScene 
                                                                        SliceTables t, VisTables v, int *work) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
@@ -1163,7 +1163,7 @@ cudaError_t cluster_vis_grid(int *blocks) {
         int sms = 0, per_sm = 0;
         g.err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (g.err == cudaSuccess)
-            g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_vis_kernel<4, 32, 7>, 128, 0);
+            g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_vis_kernel<4, 16, 7>, 128, 0);
         g.blocks = std::max(1, sms * std::max(1, per_sm));
     });
     *blocks = g.blocks;
@@ -1553,7 +1553,7 @@ rzk_status rzk_lightslice_gather(rzk_lightslice *L, const rzk_receiver *d_recv, 
         LS_TRY(cluster_vis_grid(&grid));
         const DevScene ds = L->scene->dev();
         if (v.n_items > 0)
-            cluster_vis_kernel<4, 32, 7><<<grid, 128, 0, st>>>(ds, L->d_perm.p, t, v, L->d_work.p);
+            cluster_vis_kernel<4, 16, 7><<<grid, 128, 0, st>>>(ds, L->d_perm.p, t, v, L->d_work.p);
         LS_TRY(cudaGetLastError());
         const long long threads = 32LL * t.n_items;
         cluster_shade_kernel<<<(unsigned)((threads + kShadeBlock - 1) / kShadeBlock), kShadeBlock, 0, st>>>(

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) mrcs_vis_kernel(DevScene s, 
                                                                     uint32_t *masks) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][STACK_CAP];
+    __shared__ int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
@@ -319,7 +319,7 @@ rzk_status rzk_mrcs_create(rzk_context *ctx, rzk_scene *scene, const rzk_camera 
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrcs_vis_kernel<4, 32, 5>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrcs_vis_kernel<4, 16, 7>, 128, 0);
     m->grid = std::max(1, sms * std::max(1, per_sm));
     *out = m;
     return RZK_OK;
@@ -371,7 +371,7 @@ rzk_status rzk_mrcs_gather(rzk_mrcs *m, const rzk_receiver *d_recv, int n_recv, 
     const DevScene ds = m->scene->dev();
     if (nr > 0) {
         RZK_CUDA_TRY(cudaMemsetAsync(m->work.p, 0, sizeof(int), st));
-        mrcs_vis_kernel<4, 32, 5><<<m->grid, 128, 0, st>>>(ds, d_recv, n_recv, image_width, m->reps.p, nr,
+        mrcs_vis_kernel<4, 16, 7><<<m->grid, 128, 0, st>>>(ds, d_recv, n_recv, image_width, m->reps.p, nr,
                                                            (int)wtiles, m->work.p, m->masks.p);
         RZK_CUDA_TRY(cudaGetLastError());
     }

@@ -537,6 +537,57 @@ __global__ void __launch_bounds__(256) closest_refit_kernel(int n, const float4 
 
 }  // namespace
 
+// The 8-wide any-hit tree of the packet gathers: every inner node at a depth divisible by three
+// becomes a node of up to eight entries, its descendants three levels down (or the leaves above).
+// Entry = {box min, code}, {box max, -}: code = a wide node's index, -1 - sorted triangle slot, or
+// kWideEmpty.  A parent or child index out of range (a saved tree that was damaged) is passed over.
+__global__ void wide8_parent_kernel(int nn, const float4 *tree, int *parent) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    const int c = __float_as_int(tree[2 * (i + 1)].w);
+    if (c >= 1 && c + 1 < nn) parent[c] = parent[c + 1] = i;
+}
+
+__global__ void wide8_flag_kernel(int nn, const float4 *tree, const int *parent, int *flag) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    int depth = 0;
+    for (int k = i; k > 0 && depth < 4 * STACK_CAP; ++depth) k = parent[k];
+    flag[i] = i == 0 || (__float_as_int(tree[2 * (i + 1)].w) >= 0 && depth % 3 == 0) ? 1 : 0;
+}
+
+__global__ void wide8_fill_kernel(int nn, const float4 *tree, const int *flag, const int *index, float4 *wide) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn || !flag[i]) return;
+    int node[8] = {i}, count = 1;
+    for (int round = 0; round < 3; ++round) {
+        int next[8], m = 0;
+        for (int k = 0; k < count; ++k) {
+            const int c = __float_as_int(tree[2 * (node[k] + 1)].w);
+            if (c >= 1 && c + 1 < nn) {
+                next[m++] = c;
+                next[m++] = c + 1;
+            } else {
+                next[m++] = node[k];
+            }
+        }
+        count = m;
+        for (int k = 0; k < m; ++k) node[k] = next[k];
+    }
+    float4 *rec = wide + 16 * (size_t)index[i];
+    for (int k = 0; k < 8; ++k) {
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(kWideEmpty)), hi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k < count) {
+            lo = tree[2 * (node[k] + 1)];
+            hi = tree[2 * (node[k] + 1) + 1];
+            hi.w = 0.0f;
+            if (__float_as_int(lo.w) >= 0) lo.w = __int_as_float(index[node[k]]);
+        }
+        rec[2 * k] = lo;
+        rec[2 * k + 1] = hi;
+    }
+}
+
 // Makes the closest-hit tree from the any-hit tree (on a fresh build and on a restored scene);
 // leaves the scene without one where closest hits are better off in the reference's order: no
 // any-hit tree, few triangles (36: 740 us for 4 M rays in the reference's order, 880 in this
@@ -598,6 +649,42 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
         s->device_bytes -= s->ctrav_bytes;
         s->ctrav_bytes = 0;
     }
+    return RZK_OK;
+}
+
+// Makes the packet gathers' 8-wide tree from the any-hit tree (from the reference's where there is
+// none), on a fresh build and on a restored scene.
+rzk_status build_wide_tree(rzk_scene *s, cudaStream_t st) {
+    const int nn = s->d_trav ? 2 * s->n_tris - 1 : s->n_nodes;
+    if (nn <= 0) return RZK_OK;
+    const float4 *tree = s->d_trav ? s->d_trav : s->d_nodes;
+    CallScratch mem;
+    const size_t scan_bytes = exclusive_scan_tmp_bytes(nn);
+    RZK_CUDA_TRY(mem.alloc(sizeof(int) * (3 * (size_t)nn + 64) + scan_bytes, st));
+    int *total = (int *)mem.get(), *parent = total + 64, *flag = parent + nn, *index = flag + nn;
+    const unsigned grid = (unsigned)((nn + 255) / 256);
+    RZK_CUDA_TRY(cudaMemsetAsync(parent, 0, sizeof(int) * (size_t)nn, st));
+    wide8_parent_kernel<<<grid, 256, 0, st>>>(nn, tree, parent);
+    wide8_flag_kernel<<<grid, 256, 0, st>>>(nn, tree, parent, flag);
+    RZK_CUDA_TRY(cudaGetLastError());
+    RZK_TRY(exclusive_scan_i32(flag, index, nn, total, index + nn, scan_bytes, st));
+    int n = 0;
+    RZK_CUDA_TRY(cudaMemcpyAsync(&n, total, sizeof(int), cudaMemcpyDeviceToHost, st));
+    RZK_CUDA_TRY(cudaStreamSynchronize(st));
+    if (s->n_wide8 < n) {
+        if (s->d_wide8) {
+            cudaFree(s->d_wide8);
+            s->device_bytes -= 16 * sizeof(float4) * (size_t)s->n_wide8;
+        }
+        s->d_wide8 = nullptr;
+        s->n_wide8 = 0;
+        RZK_CUDA_TRY(cudaMalloc((void **)&s->d_wide8, 16 * sizeof(float4) * (size_t)n));
+        s->n_wide8 = n;
+        s->device_bytes += 16 * sizeof(float4) * (size_t)n;
+    }
+    wide8_fill_kernel<<<grid, 256, 0, st>>>(nn, tree, flag, index, s->d_wide8);
+    RZK_CUDA_TRY(cudaGetLastError());
+    RZK_CUDA_TRY(cudaStreamSynchronize(st));
     return RZK_OK;
 }
 

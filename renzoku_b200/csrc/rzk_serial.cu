@@ -190,6 +190,7 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
     auto fail = [&](rzk_status e) {
         free_arrays(s);
         if (s->d_ctrav) cudaFree(s->d_ctrav);
+        if (s->d_wide8) cudaFree(s->d_wide8);
         delete s;
         return e;
     };
@@ -255,7 +256,8 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
     }
     for (void **p : {(void **)&s->d_v, (void **)&s->d_tp, (void **)&s->d_tri_surf})
         if (!*p && (e = cudaMalloc(p, 16)) != cudaSuccess) return fail(RZK_ERR_NOMEM);
-    const rzk_status r = build_closest_tree(s, st);
+    rzk_status r = build_closest_tree(s, st);
+    if (r == RZK_OK) r = build_wide_tree(s, st);
     if (r != RZK_OK) return fail(r);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) {
         set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
