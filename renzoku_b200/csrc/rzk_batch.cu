@@ -64,13 +64,14 @@ __device__ __forceinline__ int job_of_item(const JobTable &t, long long item) {
 }
 
 // The two-pass gather (gather_vis_kernel, gather_shade_kernel in rzk_gather.cu) over the table's
-// jobs: tracing items of t.group VPLs, then a warp per (job, tile, chunk).
+// jobs: tracing items of t.group VPLs, then a warp per (job, tile, chunk).  Without the facing
+// test: with it ten jobs of up to 192^2 x 3,000 VPLs take 24.9 ms, without 23.4.
 template <int WARPS, int TILE, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB) batch_vis_kernel(const __grid_constant__ JobTable t, int *work,
                                                                      uint32_t *masks) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][kPacketInts];
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
@@ -84,8 +85,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_vis_kernel(const __gri
         const int local = item - (int)jb.vis_begin;
         const int wt = local / n_groups;
         const int j0 = (local - wt * n_groups) * t.group, j1 = min(jb.n_vpl, j0 + t.group);
-        if (!visibility_item<TILE>(jb.s, jb.recv, jb.n_recv, jb.img_w, jb.vpls, j0, j1, wt, ws, lane,
-                                   masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0))
+        if (!visibility_item<TILE, false>(jb.s, jb.recv, jb.n_recv, jb.img_w, jb.vpls, j0, j1, wt, ws, lane,
+                                          masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0))
             break;
     }
 }
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) batch_gather_kernel(const __
                                                                         int *work) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][kPacketInts];
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);

@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_persistent_kernel(
     ChunkRing ring, float *out) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][kPacketInts];
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
@@ -505,14 +505,18 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_persistent_kernel(
 // shadow rays run as items of few VPLs, each leaving one visibility ballot per VPL, and a block
 // per (tile, chunk) then forms the marked pairs' terms in parallel and adds them in VPL order -
 // the same terms in the same order (two_pass_group says where this pays).
-template <int WARPS, int TILE, int MINB>
+// Items of up to kFaceMin VPLs go without the facing test, whose set-up per item costs more than
+// it saves there: 61 x 47 receivers x 333 VPLs, 2 an item, 107 us without and 127 with it;
+// 256^2 x 4,096 VPLs, 101 an item, 7.25 ms without and 7.01 with it.
+constexpr int kFaceMin = 4;
+template <int WARPS, int TILE, int MINB, bool FACE>
 __global__ void __launch_bounds__(WARPS * 32, MINB) gather_vis_kernel(DevScene s, const rzk_receiver *recv, int n_recv,
                                                                       int img_w, const rzk_vpl *vpls, int n_vpl,
                                                                       int group, int n_groups, int n_wtiles, int *work,
                                                                       uint32_t *masks) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][kPacketInts];
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
@@ -525,8 +529,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_vis_kernel(DevScene s
         if (item >= n_items) break;
         const int wt = item / n_groups;
         const int j0 = (item - wt * n_groups) * group, j1 = min(n_vpl, j0 + group);
-        if (!visibility_item<TILE>(s, recv, n_recv, img_w, vpls, j0, j1, wt, ws, lane,
-                                   masks + (size_t)wt * n_vpl + j0))
+        if (!visibility_item<TILE, FACE>(s, recv, n_recv, img_w, vpls, j0, j1, wt, ws, lane,
+                                         masks + (size_t)wt * n_vpl + j0))
             break;
     }
 }
@@ -977,7 +981,7 @@ static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, 
         int dev = 0, sms = 0, per_sm = 0;
         RZK_CUDA_TRY(cudaGetDevice(&dev));
         RZK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 16, 7>, 128, 0));
+        RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 16, 7, true>, 128, 0));
         ctx->vis_grid = std::max(1, sms * std::max(1, per_sm));
     }
     group = (int)std::min<long long>(kMaxGroup, std::max<long long>(1, wtiles * n_vpl / (kItems * 4 * ctx->vis_grid)));
@@ -1019,7 +1023,8 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
         const int n_groups = (n_vpl + group - 1) / group;
         RZK_CUDA_TRY(cudaMemsetAsync(ctx->d_work, 0, sizeof(int), st));
         const long long blocks = std::min<long long>(ctx->vis_grid, (wtiles * n_groups + 3) / 4);
-        gather_vis_kernel<4, 16, 7><<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, group, n_groups,
+        const auto vis = group > kFaceMin ? gather_vis_kernel<4, 16, 7, true> : gather_vis_kernel<4, 16, 7, false>;
+        vis<<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, img_w, vpls, n_vpl, group, n_groups,
                                                                       (int)wtiles, ctx->d_work, masks);
         RZK_CUDA_TRY(cudaGetLastError());
         const long long items = wtiles * n_chunks;

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) cluster_vis_kernel(DevScene 
                                                                        SliceTables t, VisTables v, int *work) {
     __shared__ __align__(128) rzk_vpl tiles[WARPS][2][TILE];
     __shared__ __align__(8) uint64_t bar[WARPS][2];
-    __shared__ int stacks[WARPS][kPacketInts];
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpStage<TILE> ws;
     ws.init(tiles[w], bar[w], stacks[w], lane);
