@@ -9,11 +9,12 @@ namespace {
 
 constexpr int kTraceBlock = 128;
 
-// The batched queries keep their lanes busy by refilling them: a warp owns a run of rays, and
-// when kRefill of its lanes have finished theirs they take the next ones together, while the
-// others go on.  One ray per thread left 6.7 (closest) and 8.4 (any hit) of 32 lanes active on
-// average, each warp waiting for its longest ray.  The traversal stack has as many entries as
-// the tree walked is deep, so that it does not limit the resident warps (64 entries: 24 per SM).
+// A query's traversal stack has as many entries as the tree walked is deep, so that it does not
+// limit the resident warps (64 entries: 24 per SM; 200,000 rays on 30k triangles 167 and 156 us).
+// Large batches in large scenes keep their lanes busy by refilling them: a warp owns a run of
+// rays, and when kRefill of its lanes have finished theirs they take the next ones together,
+// while the others go on.  One ray per thread left 6.7 (closest) and 8.4 (any hit) of 32 lanes
+// active on average there, each warp waiting for its longest ray.
 constexpr int kRefill = 8;
 
 struct RayRun {   // the warp's rays [next, end)
@@ -64,17 +65,41 @@ __global__ void __launch_bounds__(kTraceBlock) occluded_kernel(DevScene s, const
     }
 }
 
-// One ray per thread, for scenes without a closest-hit tree.
-__global__ void __launch_bounds__(kTraceBlock) closest_plain_kernel(DevScene s, const float *o, const float *d, int n,
-                                                                    float *t_out, rzk_receiver *recv) {
-    __shared__ int stack_mem[STACK_CAP * kTraceBlock];
+__global__ void __launch_bounds__(kTraceBlock) occluded_plain_kernel(GatherScene s, const float *p, const float *q,
+                                                                     int n, int cap, uint8_t *out) {
+    extern __shared__ int stack_mem[];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     Stack<kTraceBlock> stk;
-    stk.init(stack_mem + threadIdx.x);
+    stk.init(stack_mem + threadIdx.x, cap);
+    const V3 a = ld3(p + 3 * (size_t)i), b = ld3(q + 3 * (size_t)i);
+    const Ray r = make_ray(a, sub(b, a));
+    out[i] = any_hit<kTraceBlock, false, true>(s, r, s.tmin, len(sub(b, a)) - s.tmin, stk) ? 1 : 0;
+}
+
+// TREE: the scene has a closest-hit tree; otherwise cap is STACK_CAP.
+template <bool TREE>
+__global__ void __launch_bounds__(kTraceBlock) closest_plain_kernel(DevScene s, const float *o, const float *d, int n,
+                                                                    int cap, float *t_out, rzk_receiver *recv) {
+    extern __shared__ int stack_mem[];
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
     Ray r = make_ray(ld3(o + 3 * (size_t)i), ld3(d + 3 * (size_t)i));
-    float t, b, g;
-    const int slot = closest_hit<kTraceBlock>(s, r, s.tmin, RAY_TMAX, stk, &t, &b, &g);
+    float t = RAY_TMAX, b = 0.0f, g = 0.0f;
+    int slot = -1;
+    if (TREE) {
+        ClosestWalk<kTraceBlock> walk;
+        walk.stk.init(stack_mem + threadIdx.x, cap);
+        walk.start(s, r, s.tmin, RAY_TMAX);
+        while (!walk.step(s)) {}
+        int mem[STACK_CAP];   // rarely needed: local memory
+        slot = walk.template finish<1>(s, mem);
+        t = walk.bt; b = walk.bb; g = walk.bg;
+    } else if (s.n_nodes > 0) {
+        const ClosestHit c =
+            closest_in_order<kTraceBlock>(s.nodes, s.tri_isect, s.err, r, s.tmin, RAY_TMAX, stack_mem + threadIdx.x);
+        slot = c.slot; t = c.t; b = c.beta; g = c.gamma;
+    }
     if (t_out) t_out[i] = slot < 0 ? -1.0f : t;
     if (!recv) return;
     if (slot < 0) {
@@ -145,7 +170,7 @@ __global__ void __launch_bounds__(kTraceBlock) ray_query_kernel(DevScene s, cons
     rzk_ray_hit h{0, 0.0f, 0.0f, 0.0f, -1, {0, 0, 0}};
     if (closest) {
         if (s.n_nodes > 0) {
-            const ClosestHit c = closest_reference<kTraceBlock>(s.nodes, s.tri_isect, s.err, r, q.tmin, q.tmax, stk.base);
+            const ClosestHit c = closest_in_order<kTraceBlock>(s.nodes, s.tri_isect, s.err, r, q.tmin, q.tmax, stk.base);
             if (c.slot >= 0) {
                 h.hit = 1;
                 h.t = c.t;
@@ -182,7 +207,18 @@ __global__ void __launch_bounds__(kTraceBlock) primary_kernel(DevScene s, rzk_ca
 
 }  // namespace
 
-// Grid of a refilling kernel: one run of at least 32 rays per resident warp, at most kMaxRun.
+static int stack_entries(int depth) { return std::max(2, std::min(STACK_CAP, depth + 1)); }
+
+// Refilling pays where a walk is long and a lane has several rays to do; elsewhere the longest
+// ray's steps are the time and the extra work of a step only adds to them.  us on B200, one ray
+// per thread and refilled: 300k triangles 524,288 rays 586 and 515, segments 374 and 342, 200,000
+// rays 286 and 288, segments 203 and 212, 5,000 rays 129 and 142; 105k triangles 1,000,003 rays
+// 686 and 655, 524,288 390 and 378; 30k triangles 1,000,003 rays 463 and 478; 36 triangles
+// 400,000 segments 31 and 45.
+constexpr int kRefillRays = 384 << 10, kRefillTris = 64 << 10;
+
+// Grid of a refilling kernel: a run of whole warps' worth of rays per resident warp, at most
+// kMaxRun.
 struct RunGrid {
     unsigned blocks;
     int per_warp, cap;
@@ -191,7 +227,7 @@ struct RunGrid {
 template <class K>
 static cudaError_t run_grid(K kernel, int n, int depth, RunGrid &g) {
     constexpr int kMaxRun = 512;
-    g.cap = std::max(2, std::min(STACK_CAP, depth + 1));
+    g.cap = stack_entries(depth);
     g.smem = sizeof(int) * kTraceBlock * (size_t)g.cap;
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -199,7 +235,7 @@ static cudaError_t run_grid(K kernel, int n, int depth, RunGrid &g) {
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTraceBlock, g.smem);
     if (e != cudaSuccess) return e;
     const long long warps = (long long)sms * std::max(1, per_sm) * (kTraceBlock / 32);
-    g.per_warp = (int)std::min<long long>(kMaxRun, (n / warps + 31) / 32 * 32 + 32);
+    g.per_warp = (int)std::min<long long>(kMaxRun, ((n + warps - 1) / warps + 31) / 32 * 32);
     const long long runs = ((long long)n + g.per_warp - 1) / g.per_warp;
     g.blocks = (unsigned)((runs + kTraceBlock / 32 - 1) / (kTraceBlock / 32));
     return cudaSuccess;
@@ -208,6 +244,13 @@ static cudaError_t run_grid(K kernel, int n, int depth, RunGrid &g) {
 rzk_status launch_occluded(const DevScene &s, int depth, const float *p, const float *q, int n, uint8_t *out,
                            cudaStream_t st) {
     if (n <= 0) return RZK_OK;
+    if (n < kRefillRays || s.n_tris < kRefillTris) {
+        const int cap = stack_entries(depth);
+        occluded_plain_kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, sizeof(int) * kTraceBlock * cap, st>>>(
+            s, p, q, n, cap, out);
+        RZK_CUDA_TRY(cudaGetLastError());
+        return RZK_OK;
+    }
     RunGrid g;
     RZK_CUDA_TRY(run_grid(occluded_kernel, n, depth, g));
     occluded_kernel<<<g.blocks, kTraceBlock, g.smem, st>>>(s, p, q, n, g.per_warp, g.cap, out);
@@ -218,8 +261,11 @@ rzk_status launch_occluded(const DevScene &s, int depth, const float *p, const f
 rzk_status launch_closest(const DevScene &s, int depth, const float *o, const float *d, int n, float *t,
                           rzk_receiver *recv, cudaStream_t st) {
     if (n <= 0) return RZK_OK;
-    if (!s.ctrav) {
-        closest_plain_kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, st>>>(s, o, d, n, t, recv);
+    if (!s.ctrav || n < kRefillRays || s.n_tris < kRefillTris) {
+        const auto kernel = s.ctrav ? closest_plain_kernel<true> : closest_plain_kernel<false>;
+        const int cap = s.ctrav ? stack_entries(depth) : STACK_CAP;
+        kernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, sizeof(int) * kTraceBlock * cap, st>>>(s, o, d, n, cap,
+                                                                                                         t, recv);
         RZK_CUDA_TRY(cudaGetLastError());
         return RZK_OK;
     }

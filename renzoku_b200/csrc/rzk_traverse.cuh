@@ -66,11 +66,13 @@ __device__ __forceinline__ void load_pair(const float4 *p, float4 &l0, float4 &l
 // the same (see rzk_sah.cu), only the visit order differs.  FASTBOX: the ray was made by
 // make_ray, so box_hit_fast applies (1,000,003 segments on 300k triangles 571 -> 517 us, B200);
 // a caller's own ray may hold any reciprocals and takes box_hit.
-template <int STRIDE, bool STATS, bool TRAV = false, bool FASTBOX = true>
-__device__ __forceinline__ bool any_hit(const DevScene &s, const Ray &r, float tmin, float tmax,
+template <int STRIDE, bool STATS, bool TRAV = false, bool FASTBOX = true, class Scene>   // GatherScene: TRAV only
+__device__ __forceinline__ bool any_hit(const Scene &s, const Ray &r, float tmin, float tmax,
                                         Stack<STRIDE> &stk, TraceStats *ts = nullptr) {
     if (s.n_nodes == 0) return false;
-    const float4 *tree = TRAV ? s.trav : s.nodes;
+    const float4 *tree;
+    if constexpr (TRAV) tree = s.trav;
+    else tree = s.nodes;
     float4 lo = __ldg(tree + 2), hi = __ldg(tree + 3);
     if (!box_hit(lo, hi, r, tmin, tmax)) return false;
     int a = __float_as_int(lo.w);
@@ -181,11 +183,10 @@ struct ClosestHit {
 };
 
 // The reference's query: its tree, its visit order, its box test, its 64-entry stack (`stack` as
-// Stack::base).  A function of its own, so that a kernel's registers are those of closest_hit's
-// first walk.
+// Stack::base).
 template <int STRIDE>
-__device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const float4 *tri_isect, uint32_t *err,
-                                                     Ray r, float tmin, float tmax, int *stack) {
+__device__ __forceinline__ ClosestHit closest_in_order(const float4 *nodes, const float4 *tri_isect, uint32_t *err,
+                                                       const Ray &r, float tmin, float tmax, int *stack) {
     ClosestHit h{-1, RAY_TMAX, 0.0f, 0.0f};
     float4 lo = __ldg(nodes + 2), hi = __ldg(nodes + 3);
     if (!box_hit(lo, hi, r, tmin, tmax)) return h;
@@ -198,7 +199,7 @@ __device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const 
     int c = __float_as_int(lo.w);
     for (;;) {
         if (c < 0) {
-            const float4 *p = tri_isect + 3 * (size_t)(-1 - c);
+            const float4 *p = tri_isect + 3 * (-1 - c);
             float t, b, g;
             if (tri_hit<true>(__ldg(p), __ldg(p + 1), __ldg(p + 2), r, tmin, tmax, &t, &b, &g)) {
                 tmax = t;
@@ -210,8 +211,7 @@ __device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const 
             continue;
         }
         const float4 *p = nodes + 2 * (c + 1);
-        float4 l0, l1, r0, r1;
-        load_pair(p, l0, l1, r0, r1);
+        const float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
         const bool hl = box_hit(l0, l1, r, tmin, tmax);
         const bool hr = box_hit(r0, r1, r, tmin, tmax);
         if (hr) {
@@ -226,6 +226,14 @@ __device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const 
     }
     if (overflow && err) atomicOr(err, ERR_STACK);
     return h;
+}
+
+// A function of its own where it follows closest_hit's first walk, so that a kernel's registers
+// are that walk's.
+template <int STRIDE>
+__device__ __noinline__ ClosestHit closest_reference(const float4 *nodes, const float4 *tri_isect, uint32_t *err,
+                                                     Ray r, float tmin, float tmax, int *stack) {
+    return closest_in_order<STRIDE>(nodes, tri_isect, err, r, tmin, tmax, stack);
 }
 
 // The closest hit of a ray made by make_ray over [tmin, tmax]: the sorted triangle slot or -1.
