@@ -466,7 +466,7 @@ rzk_status rzk_gather_matrix(rzk_scene *s, const rzk_receiver *d_recv, int n_rec
                              void *stream) {
     if (!s || n_recv < 0 || n_vpl < 0 || (n_recv && n_vpl && !d_matrix)) return RZK_ERR_INVALID;
     if (clamp_mode < RZK_CLAMP_NONE || clamp_mode > RZK_CLAMP_RADIANCE) return RZK_ERR_INVALID;
-    return launch_matrix(s->dev(), d_recv, n_recv, d_vpls, n_vpl, clamp_mode, tau, d_matrix, d_vis, 0,
+    return launch_matrix(s->dev(), s->walk_depth(), s->box, d_recv, n_recv, d_vpls, n_vpl, clamp_mode, tau, d_matrix, d_vis, 0,
                          as_stream(stream));
 }
 
@@ -474,7 +474,7 @@ rzk_status rzk_incident_matrix(rzk_scene *s, const rzk_receiver *d_recv, int n_r
                                int n_vpl, int clamp_mode, float tau, float *d_matrix, void *stream) {
     if (!s || n_recv < 0 || n_vpl < 0 || (n_recv && n_vpl && !d_matrix)) return RZK_ERR_INVALID;
     if (clamp_mode < RZK_CLAMP_NONE || clamp_mode > RZK_CLAMP_RADIANCE) return RZK_ERR_INVALID;
-    return launch_matrix(s->dev(), d_recv, n_recv, d_vpls, n_vpl, clamp_mode, tau, d_matrix, nullptr, 1,
+    return launch_matrix(s->dev(), s->walk_depth(), s->box, d_recv, n_recv, d_vpls, n_vpl, clamp_mode, tau, d_matrix, nullptr, 1,
                          as_stream(stream));
 }
 

@@ -594,29 +594,19 @@ __global__ void reduce_chunks_kernel(const float *partial, int n_recv, int n_chu
     out[i] = acc * scale;
 }
 
-// LightTransportMatrix::fill: every pair, visibility always traced.  kind 0: radiance
-// (gather_point, lights skipped); kind 1: incident radiance without visibility; kind 2:
-// (float)visible x incident radiance, the reduced matrix of LightSlice
+// An entry of LightTransportMatrix::fill; `trace` gives the pair's visibility, always asked for
+// (but for kind 1).  kind 0: radiance (gather_point, lights skipped); kind 1: incident radiance
+// without visibility; kind 2: (float)visible x incident radiance, the reduced matrix of LightSlice
 // (lightslice.cc:721-737), with the visibility written as well.
-constexpr int kMatBlock = 128;
-__global__ void __launch_bounds__(kMatBlock) matrix_kernel(DevScene s, const rzk_receiver *recv,
-                                                           int n_recv, const rzk_vpl *vpls, int n_vpl,
-                                                           int mode, float tau, float *mat,
-                                                           uint8_t *vis, int kind) {
-    __shared__ int stack_mem[STACK_CAP * kMatBlock];
-    const int ri = blockIdx.x * kMatBlock + threadIdx.x;
-    if (ri >= n_recv) return;
-    Stack<kMatBlock> stk;
-    stk.init(stack_mem + threadIdx.x);
-    RecvRegs r = load_receiver(recv + ri);
-    for (int j = blockIdx.y; j < n_vpl; j += gridDim.y) {
-    rzk_vpl l = vpls[j];
+template <class Trace>
+__device__ __forceinline__ Rgb matrix_entry(const DevScene &s, const RecvRegs &r, const rzk_vpl &l, int mode, float tau,
+                                            int kind, bool &visible, Trace trace) {
     Rgb L = crgb(0.0f, 0.0f, 0.0f);
-    bool visible = false;
+    visible = false;
+    V3 q = ld3(l.p);
     if (kind >= 1) {
         // VirtualPointLight::incident_radiance (vpl.cc:411-440): geometric normal, no
         // visibility, surface BRDF white.
-        V3 q = ld3(l.p);
         float G = form_factor_abs(r.p, r.ng, q, ld3(l.n));
         V3 wi = unit(sub(q, r.p));
         Rgb lb = crgb(1.0f, 1.0f, 1.0f);
@@ -628,25 +618,82 @@ __global__ void __launch_bounds__(kMatBlock) matrix_kernel(DevScene s, const rzk
         L = radiance_terms(crgb(l.contrib[0], l.contrib[1], l.contrib[2]), crgb(1.0f, 1.0f, 1.0f),
                            lb, G, mode, tau);
         if (kind == 2) {
-            Ray ray = make_ray(r.p, sub(q, r.p));
-            float tmax = len(sub(q, r.p)) - s.tmin;
-            visible = !any_hit<kMatBlock, false, true>(s, ray, s.tmin, tmax, stk);
+            visible = trace(q);
             const float vf = visible ? 1.0f : 0.0f;
             L = crgb(vf * L.r, vf * L.g, vf * L.b);
         }
     } else if (r.mat >= 0) {
-        V3 q = ld3(l.p);
-        Ray ray = make_ray(r.p, sub(q, r.p));
-        float tmax = len(sub(q, r.p)) - s.tmin;
-        if (!any_hit<kMatBlock, false, true>(s, ray, s.tmin, tmax, stk)) {
-            visible = true;
+        visible = trace(q);
+        if (visible) {
             rzk_material rm = load_material(s.mats + r.mat);
             L = shade(s, r, rm, l, mode, tau, q);
         }
     }
-    size_t k = (size_t)j * n_recv + ri;
+    return L;
+}
+
+// One thread a pair, receivers fastest, with a stack as deep as the tree.  Bound by the walks'
+// dependent loads and idle lanes.  A grid of (receiver blocks x VPLs) left 124 of 384 lanes idle
+// at 260 rows, a 64-entry stack 28 of 64 warps resident: 260 x 10,007 on 300k triangles 1,544 ->
+// 975 us, 24 x 4,000 229 -> 78.
+constexpr int kMatBlock = 128;
+__global__ void __launch_bounds__(kMatBlock) matrix_kernel(DevScene s, const rzk_receiver *recv,
+                                                           int n_recv, const rzk_vpl *vpls, int n_vpl,
+                                                           int cap, int mode, float tau, float *mat,
+                                                           uint8_t *vis, int kind) {
+    extern __shared__ int stack_mem[];
+    Stack<kMatBlock> stk;
+    stk.init(stack_mem + threadIdx.x, cap);
+    const size_t k = (size_t)blockIdx.x * kMatBlock + threadIdx.x;
+    const int j = (int)(k / (unsigned)n_recv);
+    if (j >= n_vpl) return;
+    const RecvRegs r = load_receiver(recv + (int)(k - (size_t)j * n_recv));
+    const rzk_vpl &l = vpls[j];
+    bool visible;
+    const Rgb L = matrix_entry(s, r, l, mode, tau, kind, visible, [&](V3 q) {
+        Ray ray = make_ray(r.p, sub(q, r.p));
+        float tmax = len(sub(q, r.p)) - s.tmin;
+        return !any_hit<kMatBlock, false, true>(s, ray, s.tmin, tmax, stk);
+    });
     mat[3 * k] = L.r; mat[3 * k + 1] = L.g; mat[3 * k + 2] = L.b;
     if (vis) vis[k] = visible ? 1 : 0;
+}
+
+// The entries of 32 VPLs near one another (vpls: in spatial order, cols: their columns) and a run
+// of kMatRows receivers, one receiver at a time: the segments from it end close together, so they
+// are traced as a packet, and the lanes' last occluders serve the next row.  Bound by the latency
+// of a packet's steps: 260 x 10,007 pairs, 300k triangles, 81,000 packets take 650 us with 7 blocks
+// of 4 warps per SM, 688 with 5; runs of 1, 2, 4, 8 rows 729, 692, 759, 1,079 (with 5).
+constexpr int kMatRows = 2;
+template <int WARPS, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) matrix_packet_kernel(DevScene s, const rzk_receiver *recv,
+                                                                         int n_recv, const rzk_vpl *vpls,
+                                                                         const int *cols, int n_vpl, int n_runs,
+                                                                         int mode, float tau, float *mat, uint8_t *vis,
+                                                                         int kind) {
+    __shared__ __align__(16) int stacks[WARPS][kPacketInts];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long item = (long long)blockIdx.x * WARPS + w;
+    const long long group = item / n_runs;
+    if (32 * group >= n_vpl) return;
+    const int j = (int)(32 * group) + lane;
+    const bool have = j < n_vpl;
+    const rzk_vpl l = vpls[have ? j : n_vpl - 1];
+    const size_t col = (size_t)cols[have ? j : n_vpl - 1];
+    int cache = -1, cache2 = -1;
+    const int r0 = (int)(item - group * n_runs) * kMatRows, r1 = min(n_recv, r0 + kMatRows);
+    for (int ri = r0; ri < r1; ++ri) {
+        const RecvRegs r = load_receiver(recv + ri);
+        bool visible;
+        const Rgb L = matrix_entry(s, r, l, mode, tau, kind, visible, [&](V3 q) {
+            const Ray ray = make_ray(r.p, sub(q, r.p));
+            const float tmax = len(sub(q, r.p)) - s.tmin;
+            return packet_visible(s, q, r.p, ray, tmax, have, stacks[w], cache, cache2);
+        });
+        if (!have) continue;
+        const size_t k = col * n_recv + ri;
+        mat[3 * k] = L.r; mat[3 * k + 1] = L.g; mat[3 * k + 2] = L.b;
+        if (vis) vis[k] = visible ? 1 : 0;
     }
 }
 
@@ -768,7 +815,7 @@ __global__ void order_keys_kernel(const __grid_constant__ OrderTable t, uint32_t
 // VPLs 22 us and 60; at 8,192 the two are level (the work here is quadratic).
 constexpr int kRankThreads = 64, kRankTile = 1024, kRankMax = 4096;
 __global__ void __launch_bounds__(kRankThreads) order_rank_kernel(const __grid_constant__ OrderTable t,
-                                                                  const uint32_t *keys, rzk_vpl *out) {
+                                                                  const uint32_t *keys, rzk_vpl *out, int *idx) {
     __shared__ __align__(16) uint32_t sh[kRankTile];
     __shared__ int place[kRankThreads];
     const int first = blockIdx.x * kRankThreads, i = first + threadIdx.x;
@@ -796,6 +843,7 @@ __global__ void __launch_bounds__(kRankThreads) order_rank_kernel(const __grid_c
         count(own1, kRankTile, mine);
     }
     place[threadIdx.x] = before[0] + before[1] + before[2] + before[3];
+    if (i < t.total) idx[place[threadIdx.x]] = i;
     __syncthreads();
     constexpr int W = (int)(sizeof(rzk_vpl) / 16);
     const int n = min(kRankThreads, t.total - first);
@@ -865,16 +913,17 @@ int order_launches(const OrderTable &t) {
     return t.total > 0 ? 2 + radix_sort_launches(t.total, order_bits(t)) : 0;
 }
 
-rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStream_t st) {
+rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStream_t st, const int **from) {
     if (t.total <= 0) return RZK_OK;
     char *p = (char *)scratch;
     uint32_t *keys = (uint32_t *)p;
     int *idx = (int *)(p + order_up(sizeof(uint32_t) * (size_t)t.total));
     void *sort = p + 2 * order_up(sizeof(uint32_t) * (size_t)t.total);
+    if (from) *from = idx;
     order_keys_kernel<<<(t.total + 255) / 256, 256, 0, st>>>(t, keys, idx);
     RZK_CUDA_TRY(cudaGetLastError());
     if (t.total <= kRankMax) {
-        order_rank_kernel<<<(t.total + kRankThreads - 1) / kRankThreads, kRankThreads, 0, st>>>(t, keys, out);
+        order_rank_kernel<<<(t.total + kRankThreads - 1) / kRankThreads, kRankThreads, 0, st>>>(t, keys, out, idx);
         RZK_CUDA_TRY(cudaGetLastError());
         return RZK_OK;
     }
@@ -1075,12 +1124,41 @@ rzk_status ensure_scratch(rzk_context *ctx, size_t bytes) {
     return RZK_OK;
 }
 
-rzk_status launch_matrix(const DevScene &s, const rzk_receiver *recv, int n_recv, const rzk_vpl *vpls,
-                         int n_vpl, int mode, float tau, float *mat, uint8_t *vis, int kind,
+rzk_status launch_matrix(const DevScene &s, int depth, const float *box, const rzk_receiver *recv, int n_recv,
+                         const rzk_vpl *vpls, int n_vpl, int mode, float tau, float *mat, uint8_t *vis, int kind,
                          cudaStream_t st) {
     if (n_recv <= 0 || n_vpl <= 0) return RZK_OK;
-    dim3 grid((n_recv + kMatBlock - 1) / kMatBlock, std::min(n_vpl, 65535));
-    matrix_kernel<<<grid, kMatBlock, 0, st>>>(s, recv, n_recv, vpls, n_vpl, mode, tau, mat, vis, kind);
+    const size_t pairs = (size_t)n_recv * n_vpl;
+    // Packets pay where the scene is large and 32 neighbours of the VPLs' order are near one another
+    // (us, B200, one thread a pair and packets, the ordering included): 260 x 10,007 on 300k
+    // triangles 975 and 650, 75k 907 and 769, 15k 790 and 924; 260 x 4,097 on 300k 425 and 466;
+    // 96 x 4,000 194 and 403.  They need scratch, so a captured call goes without.
+    constexpr size_t kPacketPairs = 2u << 20;
+    constexpr int kPacketVpls = 8192, kPacketTris = 64 << 10;
+    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
+    if (kind != 1 && s.wide8 && s.n_tris >= kPacketTris && n_vpl >= kPacketVpls && pairs >= kPacketPairs &&
+        cudaStreamIsCapturing(st, &cap_st) == cudaSuccess && cap_st == cudaStreamCaptureStatusNone) {
+        const size_t vb = order_up(sizeof(rzk_vpl) * (size_t)n_vpl);
+        CallScratch mem;
+        if (mem.alloc(vb + order_scratch_bytes(n_vpl), st) == cudaSuccess) {
+            OrderTable t;
+            order_table_init(t);
+            order_table_add(t, vpls, n_vpl, box);
+            rzk_vpl *sorted = (rzk_vpl *)mem.get();
+            const int *cols = nullptr;
+            RZK_TRY(order_vpls(t, mem.get() + vb, sorted, st, &cols));
+            const int n_runs = (n_recv + kMatRows - 1) / kMatRows;
+            const long long blocks = ((n_vpl + 31ll) / 32 * n_runs + 3) / 4;
+            matrix_packet_kernel<4, 7><<<(unsigned)blocks, 128, 0, st>>>(s, recv, n_recv, sorted, cols, n_vpl, n_runs,
+                                                                         mode, tau, mat, vis, kind);
+            RZK_CUDA_TRY(cudaGetLastError());
+            return RZK_OK;
+        }
+        cudaGetLastError();   // no scratch: one thread a pair needs none
+    }
+    const int cap = kind == 1 ? 1 : std::max(2, std::min(STACK_CAP, depth + 1));
+    matrix_kernel<<<(unsigned)((pairs + kMatBlock - 1) / kMatBlock), kMatBlock, sizeof(int) * kMatBlock * cap, st>>>(
+        s, recv, n_recv, vpls, n_vpl, cap, mode, tau, mat, vis, kind);
     RZK_CUDA_TRY(cudaGetLastError());
     return RZK_OK;
 }

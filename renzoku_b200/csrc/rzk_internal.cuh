@@ -214,10 +214,10 @@ void order_table_init(OrderTable &t);
 bool order_table_add(OrderTable &t, const rzk_vpl *src, int n, const float *box);
 size_t order_scratch_bytes(int total);
 int order_launches(const OrderTable &t);
-rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStream_t st);
+rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStream_t st, const int **from = nullptr);
 // rzk_gather.cu: every (receiver, VPL) pair into a column-major [n_vpl][n_recv][3] matrix;
 // kind 0 radiance, 1 incident radiance, 2 visible x incident radiance (+ visibility)
-rzk_status launch_matrix(const DevScene &s, const rzk_receiver *recv, int n_recv, const rzk_vpl *vpls,
+rzk_status launch_matrix(const DevScene &s, int depth, const float *box, const rzk_receiver *recv, int n_recv, const rzk_vpl *vpls,
                          int n_vpl, int mode, float tau, float *mat, uint8_t *vis, int kind,
                          cudaStream_t st);
 // rzk_gather.cu: kernels one rzk_gather_cfg call launches

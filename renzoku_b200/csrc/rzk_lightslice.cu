@@ -1080,7 +1080,7 @@ rzk_status build(rzk_lightslice *L, const rzk_receiver *d_recv, const rzk_vpl *d
     LS_TRY(cudaGetLastError());
     LS_TRY(L->d_R.alloc(3 * (size_t)ns * n1));
     LS_TRY(L->d_V.alloc((size_t)ns * n1));
-    r = launch_matrix(sc->dev(), d_rows.p, ns, L->d_vpl1.p, n1, P.incident_clamp_mode, P.incident_tau, L->d_R.p,
+    r = launch_matrix(sc->dev(), sc->walk_depth(), sc->box, d_rows.p, ns, L->d_vpl1.p, n1, P.incident_clamp_mode, P.incident_tau, L->d_R.p,
                       L->d_V.p, 2, st);
     if (r != RZK_OK) return r;
     std::vector<float> hR(3 * (size_t)ns * n1);

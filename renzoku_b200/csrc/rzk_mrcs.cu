@@ -258,7 +258,7 @@ rzk_status rzk_mrcs_create(rzk_context *ctx, rzk_scene *scene, const rzk_camera 
     // 3. the reduced matrix (LightTransportMatrix::fill), column-major [cols][rows][3]
     DBuf<float> d_mat;
     if ((e = d_mat.alloc(3 * (size_t)rows * std::max(cols, 1))) != cudaSuccess) return fail(RZK_ERR_NOMEM);
-    rzk_status r = launch_matrix(ds, d_recv.p, rows, cols_v, cols, clamp_mode, tau, d_mat.p, nullptr, 0, st);
+    rzk_status r = launch_matrix(ds, scene->walk_depth(), scene->box, d_recv.p, rows, cols_v, cols, clamp_mode, tau, d_mat.p, nullptr, 0, st);
     if (r != RZK_OK) return fail(r);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) {
         set_last_cuda_error(e, "mrcs matrix", __FILE__, __LINE__);
