@@ -501,13 +501,13 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) gather_persistent_kernel(
 
 // The gather in two passes.  A receiver's sum over a chunk has one order, so in one pass an item
 // is a tile and a whole chunk (128 VPLs or more): milliseconds of one warp's serial work, and
-// below some billions of pairs the launch lasts as long as its longest items.  In two passes the
+// where a warp gets few of them the launch lasts as long as its longest items.  In two passes the
 // shadow rays run as items of few VPLs, each leaving one visibility ballot per VPL, and a block
 // per (tile, chunk) then forms the marked pairs' terms in parallel and adds them in VPL order -
 // the same terms in the same order (two_pass_group says where this pays).
 // Items of up to kFaceMin VPLs go without the facing test, whose set-up per item costs more than
 // it saves there: 61 x 47 receivers x 333 VPLs, 2 an item, 107 us without and 127 with it;
-// 256^2 x 4,096 VPLs, 101 an item, 7.25 ms without and 7.01 with it.
+// 256^2 x 4,096 VPLs, 96 an item, 7.25 ms without and 7.01 with it.
 constexpr int kFaceMin = 4;
 template <int WARPS, int TILE, int MINB, bool FACE>
 __global__ void __launch_bounds__(WARPS * 32, MINB) gather_vis_kernel(DevScene s, const rzk_receiver *recv, int n_recv,
@@ -1013,17 +1013,22 @@ int gather_launches(int n_recv, int n_vpl, int n_chunks) {
     return k;
 }
 
-// VPLs per tracing item of a two-pass gather, or 0 where one pass does.  Two passes are faster up
-// to some 2e9 pairs (measured to 2.7e8; us, one pass and two, B200): 61 x 47 receivers x 333 VPLs,
-// 36 triangles 657 and 96; 30k triangles 64^2 x 300 5,970 and 494, 128^2 x 3,000 11,400 and 6,850,
-// 256^2 x 3,000 17,900 and 16,300; 300k triangles 128^2 x 8,000 9,800 and 4,700; 36 triangles
-// 256^2 x 4,096 8,080 and 8,110.  At 512^2 x 32,768 (8.6e9 pairs, 300k triangles) they take 106 ms
-// to one pass's 103 and 1.07 GB of ballots.  About twenty items per resident warp even the warps'
-// loads out (3 leave a tail, 60 cost more in cold occluder caches); an item of more than 256 VPLs
-// gains nothing by being longer.
-static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, int &group) {
+// VPLs per tracing item of a two-pass gather, or 0 where one pass does.  One pass has an item per
+// (tile, chunk), and while a resident warp gets fewer than about twenty of them the launch lasts
+// as long as its longest; two passes cost more work and 4 bytes of ballots per tile and VPL.  ms in
+// one pass and two (B200; items per resident warp): 30k triangles 64^2 x 300 VPLs 3.55 and 0.28 (0.1),
+// 128^2 x 3,000 5.14 and 2.96 (3), 128^2 x 30,000 42.5 and 22.3 (4), 256^2 x 3,000 8.46 and 7.43
+// (12), 256^2 x 8,000 20.6 and 18.8 (16); 300k triangles 256^2 x 6,000 5.39 and 4.29 (16), 512^2 x
+// 1,000 2.55 and 2.43 (16), 384^2 x 3,000 4.02 and 4.22 (27), 512^2 x 8,000 13.0 and 13.8 (63),
+// 512^2 x 32,768 45.6 and 49.6 (63).  In scenes of few triangles items cost about alike and the
+// line is lower: 36 triangles 61 x 47 x 333 0.63 and 0.107 (0.1), 256^2 x 2,000 3.52 and 3.48 (8),
+// 256^2 x 3,000 5.08 and 5.16 (12), 256^2 x 4,096 6.72 and 7.01 (16).
+// About twenty tracing items per resident warp even the warps' loads out (3 leave a tail, 60 cost
+// more in cold occluder caches); an item of more than 256 VPLs gains nothing by being longer.
+static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, int n_chunks, int n_tris, int &group) {
     constexpr long long kMaskWords = 64ll << 20;   // 256 MB of ballots
     constexpr long long kItems = 20, kMaxGroup = 256;
+    constexpr int kFewTris = 128;
     group = 0;
     if (wtiles * n_vpl > kMaskWords) return RZK_OK;
     if (ctx->vis_grid == 0) {
@@ -1033,7 +1038,9 @@ static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, 
         RZK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_vis_kernel<4, 16, 7, true>, 128, 0));
         ctx->vis_grid = std::max(1, sms * std::max(1, per_sm));
     }
-    group = (int)std::min<long long>(kMaxGroup, std::max<long long>(1, wtiles * n_vpl / (kItems * 4 * ctx->vis_grid)));
+    const long long warps = 4ll * ctx->vis_grid;
+    if (wtiles * n_chunks >= (n_tris < kFewTris ? 10 : 20) * warps) return RZK_OK;
+    group = (int)std::min<long long>(kMaxGroup, std::max<long long>(1, wtiles * n_vpl / (kItems * warps)));
     if (group > 32) group = group / 32 * 32;   // whole shared-memory tiles
     return RZK_OK;
 }
@@ -1055,7 +1062,7 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     // rzk_gather_noalloc sums in measured 1.3% slower here, where memory is not short)
     const size_t plane_bytes = (sizeof(float) * 3 * (size_t)n_recv * n_chunks + 255) & ~(size_t)255;
     int group = 0;
-    if (variant == 0 && n_vpl > 0) RZK_TRY(two_pass_group(ctx, wtiles, n_vpl, group));
+    if (variant == 0 && n_vpl > 0) RZK_TRY(two_pass_group(ctx, wtiles, n_vpl, n_chunks, s.n_tris, group));
     const size_t need = plane_bytes + (group > 0 ? sizeof(uint32_t) * (size_t)wtiles * n_vpl : 0);
     if (need > ctx->partial_bytes) {
         if (ctx->d_partial) cudaFree(ctx->d_partial);
