@@ -383,7 +383,8 @@ rzk_status rzk_batch_create(rzk_context *ctx, const rzk_gather_job *jobs, int n_
                             int chunk_len, rzk_batch **out);
 /* Runs every job of the batch: one memset, then per table of up to 128 jobs the spatial
  * ordering of its chunked jobs' VPLs (as rzk_gather_cfg orders them, in one sort), one
- * persistent launch and one reduction; no allocation and no synchronisation, so it can be
+ * persistent launch (or, for a table of small jobs, a tracing and a summing launch) and one
+ * reduction; no allocation and no synchronisation, so it can be
  * captured in a CUDA graph and replayed.
  * Each job's image equals rzk_gather_cfg's for the same chunk length, bit for bit. */
 rzk_status rzk_batch_run(rzk_batch *batch, void *stream);
