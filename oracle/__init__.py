@@ -41,10 +41,10 @@ class Counters(ctypes.Structure):
 
 
 def build(ref: bool = True) -> None:
-    """Compile liboracle.so and, where the reference tree exists, _ref/librzk_ref.so and the
-    drop-in classes' driver _ref/librzk_dropin_test.so."""
+    """Compile liboracle.so and, where the reference tree exists (an empty folder in its place
+    is none), _ref/librzk_ref.so and the drop-in classes' driver _ref/librzk_dropin_test.so."""
     targets = ["oracle"]
-    if ref and os.path.isdir(REFERENCE_TREE):
+    if ref and os.path.isdir(REFERENCE_TREE) and os.listdir(REFERENCE_TREE):
         targets.append("ref")
         if os.path.exists(os.path.join(HERE, "..", "renzoku_b200", "librzk_dropin.so")):
             targets.append("dropin")

@@ -78,9 +78,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
 def build_dropin(force: bool = False) -> str | None:
     """librzk_dropin.so (renzoku_b200/dropin): the C++ classes behind the reference's
     Aggregate / IVplGenerator / Integrator interfaces.  Needs the reference's headers; where
-    they are absent the prebuilt library is used as it is (None if there is none)."""
+    they are absent (or their folder is empty) the prebuilt library is used as it is (None if
+    there is none)."""
     build()
-    if os.path.isdir(REFERENCE_TREE):
+    if os.path.isdir(REFERENCE_TREE) and os.listdir(REFERENCE_TREE):
         args = ["make", "-s", "-C", os.path.join(HERE, "dropin"), f"REF={REFERENCE_TREE}"]
         if force:
             args.append("-B")

@@ -12,6 +12,18 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200) and librzk_cuda.so")
 
 
+@pytest.fixture(scope="session", autouse=True)
+def reference_harness():
+    """A test that calls the reference harness is skipped where it could not be built."""
+    import oracle
+    if os.path.isdir(oracle.REFERENCE_TREE) and os.listdir(oracle.REFERENCE_TREE):
+        oracle.build(ref=True)
+    if not oracle.RefHarness.available():
+        def lib(cls):
+            pytest.skip("reference harness not built")
+        oracle.RefHarness.lib = classmethod(lib)
+
+
 @pytest.fixture(scope="session")
 def oracle_built():
     """Compile the CPU checkers (liboracle.so; the reference harness where the reference
