@@ -232,7 +232,7 @@ struct Shaft {
             qb[a] = qv[a] - eps;
             const float u0 = lo[a] - eps, u1 = hi[a] + eps;
             const float r0 = __fdividef(1.0f, u0), r1 = __fdividef(1.0f, u1);
-            const bool pos = u0 > 0.0f;
+            const bool pos = u0 >= 0.0f;   // at zero 1 / u0 is +inf, which bounds the exit and not the entry
             neg[a] = u1 < 0.0f;
             n1[a] = neg[a] ? 0.0f : 0.999998f * r1;
             n2[a] = pos ? 0.0f : 0.999998f * r0;
