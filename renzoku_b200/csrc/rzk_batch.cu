@@ -103,13 +103,15 @@ __global__ void __launch_bounds__(kShadeBlock) batch_shade_kernel(const __grid_c
     const int ri = lane_receiver(wt, lane, jb.n_recv, jb.img_w);
     RecvRegs r;
     rzk_material rm;
+    bool active = false;
     if (ri >= 0) {
         r = load_receiver(jb.recv + ri);
-        if (r.mat >= 0) rm = load_material(jb.s.mats + r.mat);
+        active = r.mat >= 0;
+        if (active) rm = load_material(jb.s.mats + r.mat);
     }
     const int j0 = chunk * jb.chunk_len, j1 = min(jb.n_vpl, j0 + jb.chunk_len);
-    const Rgb sum = shade_marked(jb.s, r, rm, jb.vpls, j0, j1, masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0,
-                                 jb.mode, jb.tau, lane);
+    const Rgb sum = shade_marked(jb.s, r, rm, active, jb.vpls, j0, j1,
+                                 masks + jb.mask_begin + (long long)wt * jb.n_vpl + j0, jb.mode, jb.tau, lane);
     PlaneSink{jb.partial, jb.n_recv, chunk}(ri, sum, true);
 }
 

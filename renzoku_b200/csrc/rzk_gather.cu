@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kShadeBlock) gather_shade_kernel(DevScene s, c
         if (active) rm = load_material(s.mats + r.mat);
     }
     const int j0 = chunk * chunk_len, j1 = min(n_vpl, j0 + chunk_len);
-    const Rgb sum = shade_marked(s, r, rm, vpls, j0, j1, masks + (size_t)wt * n_vpl + j0, mode, tau, lane);
+    const Rgb sum = shade_marked(s, r, rm, active, vpls, j0, j1, masks + (size_t)wt * n_vpl + j0, mode, tau, lane);
     if (ri >= 0) {
         float *o = partial + 3 * ((size_t)chunk * n_recv + ri);
         __stcs(o, sum.r); __stcs(o + 1, sum.g); __stcs(o + 2, sum.b);

@@ -702,16 +702,19 @@ __device__ __forceinline__ bool visibility_item(const GatherScene &s, const rzk_
 }
 
 // Summing half for one warp: each lane's sum, in VPL order, of its receiver's terms with the VPLs
-// of [j0, j1) that `masks` (first word: VPL j0's, from visibility_item) marks.
+// of [j0, j1) that `masks` (first word: VPL j0's, from visibility_item) marks.  A lane that is not
+// `active` (no receiver, or one without a material) adds nothing whatever its bits say: an item
+// whose bounded wait gave up leaves its words unwritten.
 __device__ __forceinline__ Rgb shade_marked(const GatherScene &s, const RecvRegs &r, const rzk_material &rm,
-                                            const rzk_vpl *vpls, int j0, int j1, const uint32_t *masks, int mode,
-                                            float tau, int lane) {
+                                            bool active, const rzk_vpl *vpls, int j0, int j1,
+                                            const uint32_t *masks, int mode, float tau, int lane) {
     Rgb sum = crgb(0.0f, 0.0f, 0.0f);
     for (int b = j0; b < j1; b += 32) {
         const uint32_t word = b + lane < j1 ? __ldcs(masks + (b - j0) + lane) : 0u;
         for (unsigned todo = __ballot_sync(kFull, word != 0u); todo; todo &= todo - 1u) {
             const int v = __ffs(todo) - 1;
-            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
+            const bool marked = (__shfl_sync(kFull, word, v) >> lane) & 1u;
+            if (!marked || !active) continue;
             const rzk_vpl l = load_vpl(vpls + b + v);
             sum = cadd(sum, pair_radiance(s, r, rm, l, pair_geo(r, l), mode, tau));
         }
@@ -722,7 +725,8 @@ __device__ __forceinline__ Rgb shade_marked(const GatherScene &s, const RecvRegs
 // Summing half with one order of additions per sum but the terms formed in parallel: the warps
 // of a block (at least three) take the VPLs of [j0, j1) in turn, 32 VPLs at a time, and leave the
 // terms in `terms`; then thread t < 96 adds channel t / 32 of receiver t % 32 in VPL order.
-// Returns that thread's sum.  `masks` as from visibility_item, its first word VPL j0's.
+// Returns that thread's sum.  `masks` as from visibility_item, its first word VPL j0's; `active` as
+// in shade_marked.
 template <int WARPS>
 __device__ __forceinline__ float shade_chunk(const GatherScene &s, const RecvRegs &r, bool active, const rzk_vpl *vpls,
                                              int j0, int j1, const uint32_t *masks, int mode, float tau,
@@ -738,7 +742,8 @@ __device__ __forceinline__ float shade_chunk(const GatherScene &s, const RecvReg
         for (unsigned todo = some; todo; todo &= todo - 1u, ++k) {
             if (k % WARPS != w) continue;
             const int v = __ffs(todo) - 1;
-            if (!((__shfl_sync(kFull, word, v) >> lane) & 1u)) continue;
+            const bool marked = (__shfl_sync(kFull, word, v) >> lane) & 1u;
+            if (!marked || !active) continue;
             const rzk_vpl l = load_vpl(vpls + b + v);
             const PairGeo pg = pair_geo(r, l);
             const Rgb L = pair_radiance(s, r, load_material(s.mats + r.mat), l, pg, mode, tau);
@@ -750,7 +755,8 @@ __device__ __forceinline__ float shade_chunk(const GatherScene &s, const RecvReg
         if (w < 3) {
             for (unsigned todo = some; todo; todo &= todo - 1u) {
                 const int v = __ffs(todo) - 1;
-                if ((__shfl_sync(kFull, word, v) >> lane) & 1u) acc += terms[v][w][lane];
+                const bool marked = (__shfl_sync(kFull, word, v) >> lane) & 1u;
+                if (marked && active) acc += terms[v][w][lane];
             }
         }
         __syncthreads();
