@@ -393,15 +393,22 @@ __device__ __forceinline__ bool packet_visible(const GatherScene &s, V3 p, V3 q,
 // q - p, and with both taken relative to a point c of the tile
 //   n_r . (q - p)  = (n_r, -n_r . (p - c)) . (q - c, 1)
 //   nn_v . (q - p) = (p - c, 1) . (-nn_v, nn_v . (q - c))
-// so the two tests of a block are two products with an inner dimension of 4 (tf32, operands as
-// they are: the low 13 bits are ignored).  A pair is dropped only where a product is past zero by
-// more than 2.4e-3 (|q - c| + R) + 1e-8, R the largest |p - c|: the truncated operands are within
-// 2^-10 of themselves, so a product of unit normals is within 1.98e-3 |q - c| + 1e-3 R (or the
-// other way round), and what is left bounds the rounding of the exact test and keeps |q - p|
-// above 1e-8; normals that are not unit vectors, powers that are not finite and coordinates past
-// 1e8 drop nothing (an infinite margin, which no product is past).  Every dropped pair fails pair_survives, which decides the others, so the
-// surviving pairs are the same.  The division-free test it replaces took about 55 instructions a
-// VPL, this about 12: 512^2 x 32,768 VPLs 61.0 -> 45.8 ms, its clustered gather 7.1 -> 6.7.
+// so the two tests of a block are two products with an inner dimension of 4 (operands rounded to
+// tf32).  A pair is dropped only where a product is past zero by more than
+// 2.4e-3 (|q - c| + R) + 1e-8, R the largest |p - c|: the rounded operands are within 2^-11 of
+// themselves, so a product of unit normals is within 1e-3 |q - c| + 0.5e-3 R (or the other way
+// round), and what is left bounds the rounding of the exact test and keeps |q - p| above 1e-8;
+// normals that are not unit vectors, powers that are not finite and coordinates past 1e8 drop
+// nothing (an infinite margin, which no product is past).  Every dropped pair fails pair_survives,
+// which decides the others, so the surviving pairs are the same.  The division-free test it
+// replaces took about 55 instructions a VPL, this about 12: 512^2 x 32,768 VPLs 61.0 -> 45.8 ms,
+// its clustered gather 7.1 -> 6.7.
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return r;
+}
+
 struct FaceTest {
     uint32_t a1[4], a2[4];   // rows g and g + 8 of the two 16-receiver blocks, component lane % 4
     V3 c;
@@ -423,8 +430,8 @@ struct FaceTest {
                         n2 = __shfl_sync(kFull, n.z, row), n3 = __shfl_sync(kFull, k1, row);
             const float x0 = __shfl_sync(kFull, x.x, row), x1 = __shfl_sync(kFull, x.y, row),
                         x2 = __shfl_sync(kFull, x.z, row);
-            a1[i] = __float_as_uint(t == 0 ? n0 : t == 1 ? n1 : t == 2 ? n2 : n3);
-            a2[i] = __float_as_uint(t == 0 ? x0 : t == 1 ? x1 : t == 2 ? x2 : 1.0f);
+            a1[i] = to_tf32(t == 0 ? n0 : t == 1 ? n1 : t == 2 ? n2 : n3);
+            a2[i] = to_tf32(t == 0 ? x0 : t == 1 ? x1 : t == 2 ? x2 : 1.0f);
         }
     }
     // bit v of the result: this lane's receiver may have a term with VPL v of `vpls` (shared
@@ -448,8 +455,8 @@ struct FaceTest {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const rzk_vpl &l = vpls[8 * h + g];
-            const float b1 = t < 3 ? l.p[t < 3 ? t : 0] - ct : 1.0f;
-            const float b2 = t < 3 ? -l.nn[t < 3 ? t : 0] : margin[8 * h + g].x;
+            const uint32_t b1 = to_tf32(t < 3 ? l.p[t < 3 ? t : 0] - ct : 1.0f);
+            const uint32_t b2 = to_tf32(t < 3 ? -l.nn[t < 3 ? t : 0] : margin[8 * h + g].x);
             const float4 m0 = margin[8 * h + 2 * t], m1 = margin[8 * h + 2 * t + 1];
             const uint32_t bit = 1u << (8 * h + 2 * t);
 #pragma unroll
@@ -457,10 +464,10 @@ struct FaceTest {
                 float d[4], e[4];
                 asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                    : "r"(a1[2 * i]), "r"(a1[2 * i + 1]), "r"(__float_as_uint(b1)), "f"(0.0f));
+                    : "r"(a1[2 * i]), "r"(a1[2 * i + 1]), "r"(b1), "f"(0.0f));
                 asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
                     : "=f"(e[0]), "=f"(e[1]), "=f"(e[2]), "=f"(e[3])
-                    : "r"(a2[2 * i]), "r"(a2[2 * i + 1]), "r"(__float_as_uint(b2)), "f"(0.0f));
+                    : "r"(a2[2 * i]), "r"(a2[2 * i + 1]), "r"(b2), "f"(0.0f));
                 if (!(d[0] < -m0.y) && !(e[0] > m0.z)) rows[i] |= bit;
                 if (!(d[1] < -m1.y) && !(e[1] > m1.z)) rows[i] |= bit << 1;
                 if (!(d[2] < -m0.y) && !(e[2] > m0.z)) rows[i] |= bit << 16;

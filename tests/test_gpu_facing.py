@@ -63,3 +63,28 @@ def test_far_positions_drop_nothing(ctx, far):
         (_, want, _), *rest = _images(ctx, agg, recv, rzk.records_to_device(vpls))
         for variant, got, _ in rest:
             assert np.array_equal(got, want, equal_nan=True), (place, variant)
+
+
+@pytest.mark.parametrize("kind,scale,shift", [("room", 1, 0), ("objects", 1, 0), ("objects", 0.02, 0), ("objects", 300, 0),
+                                              ("objects", 1, 70), ("spheres", 5, -900)])
+def test_units_and_places(ctx, kind, scale, shift):
+    from renzoku_b200 import rzk
+    sc = {"room": lambda: sg.room_boxes(SIDE, SIDE), "spheres": lambda: sg.room_spheres(300, SIDE, SIDE, seed=6),
+          "objects": lambda: sg.room_objects(150, SIDE, SIDE, seed_geo=51, seed_mat=52)}[kind]()
+    v = sc.prim_v.reshape(-1, 4, 3) * np.float32(scale) + np.float32(shift)
+    cam = dataclasses.replace(sc.camera, eye=tuple(scale * x + shift for x in sc.camera.eye),
+                              lookat=tuple(scale * x + shift for x in sc.camera.lookat))
+    agg = rzk.AggregateCuda(ctx, dataclasses.replace(sc, prim_v=np.ascontiguousarray(v.reshape(-1, 12)), camera=cam))
+    recv = agg.primary(rzk.Camera(cam))
+    rec = rzk.records_from_device(recv, sg.RECEIVER_DTYPE)
+    rng = np.random.default_rng(8)
+    vpls = _surface_vpls(rec[rec["mat"] >= 0], rng)
+    vpls["p"][::7] += rng.normal(0, 0.3 * scale, (N_VPL, 3))[::7]   # off the surfaces
+    vpls["p"][::50] += 4 * scale                                    # and outside the scene
+    vpls["mat"][::5] = -1
+    images = _images(ctx, agg, recv, rzk.records_to_device(vpls))
+    rays = images[1][2]
+    assert 0 < rays < SIDE * SIDE * N_VPL
+    for variant, got, n in images[1:]:
+        # a receiver at a VPL has a NaN term; everything else is the same number
+        assert np.array_equal(got, images[0][1], equal_nan=True) and n == rays, variant
