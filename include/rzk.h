@@ -226,8 +226,8 @@ rzk_status rzk_scene_serialized_size(rzk_scene *scene, size_t *bytes);
  * bytes used.  Synchronises `stream`. */
 rzk_status rzk_scene_serialize(rzk_scene *scene, void *h_buf, size_t cap, size_t *written, void *stream);
 /* A new scene on ctx's device from a blob; RZK_ERR_INVALID for a blob that is not one (bad
- * magic or version, truncated, sizes that disagree with its counts).  Synchronises
- * `stream`. */
+ * magic or version, truncated, sizes that disagree with its counts, a tree whose links or
+ * triangles are out of range).  Synchronises `stream`. */
 rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t size, void *stream,
                                  rzk_scene **out);
 

@@ -142,6 +142,29 @@ rzk_status write_scene(rzk_scene *s, Writer &w, cudaStream_t st, bool copy) {
     return RZK_OK;
 }
 
+// Whether a blob's packed tree of nn nodes over n triangles is one: every inner node's children
+// are a pair of later nodes that no other node has, every node but the root is such a child, and
+// every leaf names a triangle.  The kernels that derive trees from it, and the walks, follow its
+// codes unchecked.  depth = of its deepest node.  `nodes` need not be aligned.
+bool tree_ok(const char *nodes, int64_t nn, int n, int &depth) {
+    std::vector<int> at((size_t)nn, -1);
+    depth = 0;
+    if (nn > 0) at[0] = 0;
+    for (int64_t i = 0; i < nn; ++i) {
+        if (at[i] < 0) return false;
+        depth = std::max(depth, at[i]);
+        int32_t code;
+        std::memcpy(&code, nodes + 32 * (i + 1) + 12, sizeof(code));
+        if (code < 0) {
+            if (-1 - code >= n) return false;
+        } else {
+            if (code <= i || (int64_t)code + 1 >= nn || at[code] >= 0 || at[code + 1] >= 0) return false;
+            at[code] = at[code + 1] = at[i] + 1;
+        }
+    }
+    return true;
+}
+
 void free_arrays(rzk_scene *s) {
     for (const Array &a : scene_arrays(s))
         if (*a.ptr) { cudaFree(*a.ptr); *a.ptr = nullptr; }
@@ -209,7 +232,8 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
         return fail(RZK_ERR_INVALID);
     // every array's recorded size must be 0 or the size its counts give
     std::vector<Array> arrays = scene_arrays(s);
-    // d_wide and d_trav are sized by the blob (held only when the source scene built them)
+    if ((int64_t)h.n_nodes > 2 * (int64_t)h.n_tris) return fail(RZK_ERR_INVALID);
+    // d_wide and d_trav are held only when the source scene built them
     std::vector<uint64_t> sizes(arrays.size());
     std::vector<size_t> offs(arrays.size());
     for (size_t k = 0; k < arrays.size(); ++k) {
@@ -219,8 +243,12 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
         rd.off += (size_t)sizes[k];
     }
     if (h.n_arrays != arrays.size() || rd.off != size) return fail(RZK_ERR_INVALID);
-    for (size_t k = 0; k < arrays.size(); ++k)   // no any-hit tree in the blob: none here either
-        if (arrays[k].ptr == (void **)&s->d_trav && sizes[k] == 0) s->trav_bytes = 0;
+    const size_t full = sizeof(float4) * 4 * (size_t)h.n_tris;   // build_sah_tree's 2 n - 1 nodes and slot 0
+    for (size_t k = 0; k < arrays.size(); ++k)
+        if (arrays[k].ptr == (void **)&s->d_trav) {
+            if (sizes[k] != 0 && s->trav_bytes != full) return fail(RZK_ERR_INVALID);
+            if (sizes[k] == 0) s->trav_bytes = 0;   // no any-hit tree in the blob: none here either
+        }
     const size_t wide_bytes = sizeof(float4) * 8 * (size_t)std::max(1, h.n_wide);
     for (size_t k = 0; k < arrays.size(); ++k) {
         const bool is_wide = arrays[k].ptr == (void **)&s->d_wide, is_trav = arrays[k].ptr == (void **)&s->d_trav;
@@ -228,13 +256,36 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
         if (sizes[k] != 0 && sizes[k] != expect) return fail(RZK_ERR_INVALID);
         if (sizes[k] == 0 && expect != 0 && !is_wide && !is_trav) return fail(RZK_ERR_INVALID);
     }
+    // what the restore's own kernels and the walks index with
+    const char *base = (const char *)h_buf;
+    for (size_t k = 0; k < arrays.size(); ++k) {
+        if (sizes[k] == 0) continue;
+        const char *p = base + offs[k];
+        int depth = 0;
+        if (arrays[k].ptr == (void **)&s->d_nodes && !tree_ok(p, h.n_nodes, h.n_tris, depth)) return fail(RZK_ERR_INVALID);
+        if (arrays[k].ptr == (void **)&s->d_trav) {
+            if (!tree_ok(p, 2 * (int64_t)h.n_tris - 1, h.n_tris, depth)) return fail(RZK_ERR_INVALID);
+            s->trav_depth = depth;   // sizes the walks' stacks
+        }
+        if (arrays[k].ptr == (void **)&s->d_perm)
+            for (int i = 0; i < h.n_tris; ++i) {
+                int32_t t;
+                std::memcpy(&t, p + sizeof(t) * (size_t)i, sizeof(t));
+                if (t < 0 || t >= h.n_tris) return fail(RZK_ERR_INVALID);
+            }
+        if (arrays[k].ptr == (void **)&s->d_lights)
+            for (int i = 0; i < h.n_lights; ++i) {
+                DevLight l;
+                std::memcpy(&l, p + sizeof(l) * (size_t)i, sizeof(l));
+                if (l.n_tris < 1 || l.n_tris > 2) return fail(RZK_ERR_INVALID);
+            }
+    }
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) {
         set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
         return fail(RZK_ERR_CUDA);
     }
-    const char *base = (const char *)h_buf;
     for (size_t k = 0; k < arrays.size(); ++k) {
         if (sizes[k] == 0) continue;
         // the surfaces and materials were always allocated (16 bytes when empty)
