@@ -8,7 +8,9 @@
 // leaf box = the triangle's box (the reference's leaf box, aggregate_bvh.cc:183-209) and
 // inner box = the exact union of its children therefore returns the reference's visibility
 // bit for bit; a tree with less overlap than the Morton LBVH simply reaches the answer in
-// fewer steps.  Closest-hit queries keep the reference tree, whose visit order decides ties.
+// fewer steps.  Closest hits walk this tree's nodes in inflated boxes (below) and go back to the
+// reference tree, whose visit order decides ties, only where a tie is possible or those boxes do
+// not cover the ray.
 //
 // Binned SAH: 32 bins on the centroid axis of largest extent; past depth 32 or when no split
 // separates the centroids, the median of the Morton order the slots came in.  Nodes are
@@ -732,7 +734,7 @@ rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st) {
         RZK_CUDA_TRY(cudaGetLastError());
         // a level has nodes only if the one before it had: look once in four levels, the first
         // time when an even split would be done
-        if ((level & 3) == 3 && (kSmall << level) >= n) {
+        if ((level & 3) == 3 && (level >= 23 || (kSmall << level) >= n)) {   // past 2^30: any n
             RZK_CUDA_TRY(cudaMemcpyAsync(&pending, n_large + level + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
             RZK_CUDA_TRY(cudaStreamSynchronize(st));
         }
