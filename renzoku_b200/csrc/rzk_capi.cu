@@ -150,6 +150,8 @@ rzk_status rzk_context_destroy(rzk_context *c) {
     if (c->d_stage) cudaFree(c->d_stage);
     if (c->d_work) cudaFree(c->d_work);
     if (c->d_order) cudaFree(c->d_order);
+    for (uint32_t *m : c->d_masks)
+        if (m) cudaFree(m);
     pool_context_destroyed(c->device);
     delete c;
     return RZK_OK;

@@ -1026,7 +1026,7 @@ int gather_launches(int n_recv, int n_vpl, int n_chunks) {
 // About twenty tracing items per resident warp even the warps' loads out (3 leave a tail, 60 cost
 // more in cold occluder caches); an item of more than 256 VPLs gains nothing by being longer.
 static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, int n_chunks, int n_tris, int &group) {
-    constexpr long long kMaskWords = 64ll << 20;   // 256 MB of ballots
+    constexpr long long kMaskWords = 1ll << rzk_context::kMaskLogMax;
     constexpr long long kItems = 20, kMaxGroup = 256;
     constexpr int kFewTris = 128;
     group = 0;
@@ -1045,6 +1045,23 @@ static rzk_status two_pass_group(rzk_context *ctx, long long wtiles, int n_vpl, 
     return RZK_OK;
 }
 
+// The context's smallest buffer of at least `words` ballots, made where it has none.  Null, and the
+// gather runs in one pass, where there is no memory for it or the stream is being captured (no
+// allocation then; a gather of this size before the capture leaves the buffer).
+static uint32_t *mask_buffer(rzk_context *ctx, long long words, cudaStream_t st) {
+    int first = 0;
+    while ((1ll << (rzk_context::kMaskLog0 + first)) < words) ++first;
+    for (int k = first; k <= rzk_context::kMaskLogMax - rzk_context::kMaskLog0; ++k)
+        if (ctx->d_masks[k]) return ctx->d_masks[k];
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+        cudaMalloc((void **)&ctx->d_masks[first], sizeof(uint32_t) << (rzk_context::kMaskLog0 + first)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->d_masks[first] = nullptr;
+    }
+    return ctx->d_masks[first];
+}
+
 rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, const rzk_receiver *recv,
                          int n_recv, int img_w, const rzk_vpl *vpls, int n_vpl, int mode, float tau,
                          float scale, float *out, int variant, int n_chunks, cudaStream_t st) {
@@ -1060,10 +1077,10 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     resolve_chunks(n_vpl, n_chunks, chunk_len);
     // one plane of partial sums per chunk, added by reduce_chunks_kernel (the chunk ring that
     // rzk_gather_noalloc sums in measured 1.3% slower here, where memory is not short)
-    const size_t plane_bytes = (sizeof(float) * 3 * (size_t)n_recv * n_chunks + 255) & ~(size_t)255;
+    const size_t need = sizeof(float) * 3 * (size_t)n_recv * n_chunks;
     int group = 0;
     if (variant == 0 && n_vpl > 0) RZK_TRY(two_pass_group(ctx, wtiles, n_vpl, n_chunks, s.n_tris, group));
-    const size_t need = plane_bytes + (group > 0 ? sizeof(uint32_t) * (size_t)wtiles * n_vpl : 0);
+    uint32_t *masks = group > 0 ? mask_buffer(ctx, wtiles * n_vpl, st) : nullptr;
     if (need > ctx->partial_bytes) {
         if (ctx->d_partial) cudaFree(ctx->d_partial);
         ctx->d_partial = nullptr;
@@ -1074,8 +1091,7 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     if (!ctx->d_work) RZK_CUDA_TRY(cudaMalloc((void **)&ctx->d_work, 64));
     float *part = ctx->d_partial;
     if (n_chunks > 1) RZK_TRY(order_gather_vpls(ctx, box, vpls, n_vpl, &vpls, st));
-    if (group > 0) {
-        uint32_t *masks = (uint32_t *)((char *)part + plane_bytes);
+    if (masks) {
         const int n_groups = (n_vpl + group - 1) / group;
         RZK_CUDA_TRY(cudaMemsetAsync(ctx->d_work, 0, sizeof(int), st));
         const long long blocks = std::min<long long>(ctx->vis_grid, (wtiles * n_groups + 3) / 4);

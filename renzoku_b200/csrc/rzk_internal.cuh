@@ -117,6 +117,10 @@ struct rzk_context {
     size_t order_bytes = 0;
     int persistent_grid[16] = {0};
     int vis_grid = 0;   // resident grid of the two-pass gather's tracing kernel
+    // ballots of two-pass gathers: buffer k holds 2^(kMaskLog0 + k) words.  None is freed before
+    // the context is, so that a captured gather stays good whatever gathers run after it.
+    static constexpr int kMaskLog0 = 16, kMaskLogMax = 26;   // 256 KB to 256 MB
+    uint32_t *d_masks[kMaskLogMax - kMaskLog0 + 1] = {};
 };
 
 struct rzk_scene {
