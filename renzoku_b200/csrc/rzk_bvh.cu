@@ -561,6 +561,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
                                             s->d_nbmin, s->d_nbmax, s->d_wide);
         RZK_CUDA_TRY(cudaGetLastError());
     }
+    mem.release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     // the any-hit traversal tree (rzk_sah.cu); without it any-hit walks the reference tree
     if (s->build_trav) {

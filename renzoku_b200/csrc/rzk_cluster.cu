@@ -318,6 +318,10 @@ struct DevBuf {
         p = (T *)mem.get();
         return e;
     }
+    void release() {
+        mem.release();
+        p = nullptr;
+    }
 };
 
 }  // namespace
@@ -336,6 +340,7 @@ static rzk_status column_stats_and_alphas(const float *mat, int rows, int cols, 
     rowsum_kernel<<<(rows + kRowTile - 1) / kRowTile + 1, kRowThreads, 0, st>>>(mat, rows, cols, u, rmag, c0);
     column_kernel<true><<<grid, kStatThreads, 0, st>>>(mat, rows, cols, rmag, nullptr, nullptr, u, c0, alphas);
     RZK_CUDA_TRY(cudaGetLastError());
+    buf.release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     return RZK_OK;
 }
@@ -425,6 +430,8 @@ rzk_status cluster_by_sampling(const float *mat, int rows, int cols, int num_clu
     std::vector<float> mags(cols);
     RZK_CUDA_TRY(cudaMemcpyAsync(owner.data(), d_owner.p, sizeof(int) * cols, cudaMemcpyDeviceToHost, st));
     RZK_CUDA_TRY(cudaMemcpyAsync(mags.data(), nm.p, sizeof(float) * cols, cudaMemcpyDeviceToHost, st));
+    for (DevBuf<float> *b : {&alphas, &nm, &d_w, &K, &kn, &D}) b->release();
+    for (DevBuf<int> *b : {&d_cen, &d_owner}) b->release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     if (h_mags) std::copy(mags.begin(), mags.end(), h_mags);
     // members in column order, pdf over magnitudes, representative (cluster_builder.cc:228-272)

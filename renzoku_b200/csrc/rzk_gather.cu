@@ -1197,6 +1197,7 @@ rzk_status launch_mean(rzk_context *ctx, const DevScene &s, const rzk_receiver *
     mean_kernel<<<nb, kMeanBlock, 0, st>>>(s, recv, n_recv, vpls, n_vpl, seed, n_pairs, buf + 1);
     mean_final_kernel<<<1, 32, 0, st>>>(buf + 1, nb, n_pairs, buf);
     cudaError_t e = cudaMemcpyAsync(h_mean, buf, sizeof(double), cudaMemcpyDeviceToHost, st);
+    mem.release();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { set_last_cuda_error(e, "mean", __FILE__, __LINE__); return RZK_ERR_CUDA; }
     (void)ctx;

@@ -27,17 +27,21 @@ void set_last_cuda_error(cudaError_t e, const char *what, const char *file, int 
 // A cudaMalloc and cudaFree pair costs 100-400 us each and waits for the whole device (VPL
 // generation of the 24,000-particle frame: 0.64 of 1.1 ms; clustering 10,000 columns: 1.8 of
 // 2.6 ms; many milliseconds now and then); from the pool it is a few microseconds.  The pool
-// keeps at most kPoolKeep bytes that no call uses, serves any number of threads and streams
-// (the runtime orders reuse across streams), and is emptied when the device's last context is
-// destroyed.
+// serves any number of threads and streams (the runtime orders reuse across streams).  What it
+// holds beyond kPoolKeep without a call using it goes back to the device when a stream is next
+// waited for, so a call that waits releases its scratch before it does.  It is emptied when the
+// device's last context is destroyed, and not destroyed with it: another thread's call may be using
+// it (destroying it then crashed the process).
 constexpr unsigned long long kPoolKeep = 256ull << 20;
 class CallScratch {
 public:
     CallScratch() = default;
     CallScratch(const CallScratch &) = delete;
     CallScratch &operator=(const CallScratch &) = delete;
-    ~CallScratch() {
+    ~CallScratch() { release(); }
+    void release() {   // after the last kernel that uses the memory has been launched
         if (p_) cudaFreeAsync(p_, st_);
+        p_ = nullptr;
     }
     cudaError_t alloc(size_t bytes, cudaStream_t st);   // once per object, on the current device
     char *get() const { return (char *)p_; }

@@ -642,6 +642,7 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
         RZK_CUDA_TRY(cudaGetLastError());
         double h[2];
         RZK_CUDA_TRY(cudaMemcpyAsync(h, cost, sizeof(h), cudaMemcpyDeviceToHost, st));
+        mem.release();
         RZK_CUDA_TRY(cudaStreamSynchronize(st));
         if (h[1] <= kMaxInflation * h[0]) return RZK_OK;
     }
@@ -686,6 +687,7 @@ rzk_status build_wide_tree(rzk_scene *s, cudaStream_t st) {
     }
     wide8_fill_kernel<<<grid, 256, 0, st>>>(nn, tree, flag, index, s->d_wide8);
     RZK_CUDA_TRY(cudaGetLastError());
+    mem.release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     return RZK_OK;
 }
@@ -743,6 +745,7 @@ rzk_status build_sah_tree(rzk_scene *s, cudaStream_t st) {
         box, idx0, idx1, small, n_small, s->d_trav, max_depth);
     RZK_CUDA_TRY(cudaGetLastError());
     RZK_CUDA_TRY(cudaMemcpyAsync(&s->trav_depth, max_depth, sizeof(int), cudaMemcpyDeviceToHost, st));
+    mem.release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     return s->trav_depth >= STACK_CAP - 2 ? RZK_ERR_STACK : RZK_OK;
 }

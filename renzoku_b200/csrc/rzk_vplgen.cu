@@ -260,6 +260,7 @@ rzk_status launch_vplgen(rzk_scene *sc, uint32_t seed, int n_particles, int max_
     if (e != RZK_OK) return e;
     compact_kernel<<<(n_particles + 127) / 128, 128, 0, st>>>(slots, counts, offs, n_particles, per, out, cap);
     RZK_CUDA_TRY(cudaGetLastError());
+    mem.release();
     RZK_CUDA_TRY(cudaStreamSynchronize(st));
     return RZK_OK;
 }
