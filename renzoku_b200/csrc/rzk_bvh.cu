@@ -447,6 +447,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
     size_t scratch_bytes = 0;
     auto carve = [&](size_t bytes) { size_t off = scratch_bytes; scratch_bytes += (bytes + 255) & ~(size_t)255; return off; };
     size_t o_keys2 = carve(sizeof(uint32_t) * (size_t)n);
+    size_t o_vals = carve(sizeof(int) * (size_t)n);
     size_t o_vals2 = carve(sizeof(int) * (size_t)n);
     size_t o_hist = carve(sizeof(int) * (size_t)hist_n);
     size_t o_offs = carve(sizeof(int) * (size_t)hist_n);
@@ -460,7 +461,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
     RZK_CUDA_TRY(mem.alloc(scratch_bytes, st));
     char *scratch = mem.get();
     uint32_t *keys2 = (uint32_t *)(scratch + o_keys2);
-    int *vals2 = (int *)(scratch + o_vals2);
+    int *vals = (int *)(scratch + o_vals), *vals2 = (int *)(scratch + o_vals2);
     int *hist = (int *)(scratch + o_hist);
     int *offs = (int *)(scratch + o_offs);
     int *split = (int *)(scratch + o_split);
@@ -478,14 +479,16 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
     box_reduce_kernel<<<rb, 256, 0, st>>>(s->d_bmin, s->d_bmax, n, box + 6);
     box_final_kernel<<<1, 32, 0, st>>>(box + 6, rb, box);
     RZK_CUDA_TRY(cudaMemcpyAsync(s->box, box, sizeof(float) * 6, cudaMemcpyDeviceToHost, st));
-    morton_kernel<<<grid, TB, 0, st>>>(s->d_bmin, s->d_bmax, n, box, s->d_codes, s->d_perm);
+    morton_kernel<<<grid, TB, 0, st>>>(s->d_bmin, s->d_bmax, n, box, s->d_codes, vals);
     RZK_CUDA_TRY(cudaGetLastError());
 
-    // K2: four 8-bit passes; the data ends in d_sorted_codes / d_perm after an even count
+    // K2: four 8-bit passes; the data ends in d_sorted_codes / vals after an even count.  What the
+    // queries read is written once, with its final values: a rebuild writes the bytes that are
+    // there already, and queries on other streams go on meanwhile.
     RZK_CUDA_TRY(cudaMemcpyAsync(s->d_sorted_codes, s->d_codes, sizeof(uint32_t) * n,
                                  cudaMemcpyDeviceToDevice, st));
     uint32_t *ka = s->d_sorted_codes, *kb = keys2;
-    int *va = s->d_perm, *vb = vals2;
+    int *va = vals, *vb = vals2;
     for (int pass = 0; pass < 4; ++pass) {
         int shift = 8 * pass;
         radix_hist_kernel<<<nblocks_sort, kSortThreads, 0, st>>>(ka, n, shift, hist, nblocks_sort);
@@ -495,6 +498,7 @@ rzk_status bvh_build(rzk_scene *s, cudaStream_t st) {
         std::swap(ka, kb);
         std::swap(va, vb);
     }
+    RZK_CUDA_TRY(cudaMemcpyAsync(s->d_perm, va, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
     RZK_CUDA_TRY(cudaGetLastError());
 
     // K3: BFS levels; the host needs each level's size to size the next launch

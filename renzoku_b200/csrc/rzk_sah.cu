@@ -621,6 +621,8 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
             RZK_CUDA_TRY(cudaMalloc((void **)&s->d_ctrav, bytes));
             s->ctrav_bytes = bytes;
             s->device_bytes += bytes;
+            // slot 0; the kernels write every node (not cleared on a rebuild: queries may be reading)
+            RZK_CUDA_TRY(cudaMemsetAsync(s->d_ctrav, 0, 2 * sizeof(float4), st));
         }
         const float radius = 2.0f * ext;   // the covered origins: a sphere about the scene's centre
         Inflate inf;
@@ -635,7 +637,6 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
         int *count = (int *)(cost + 2), *parent = count + nn;
         RZK_CUDA_TRY(cudaMemsetAsync(cost, 0, 2 * sizeof(double) + sizeof(int) * nn, st));
         RZK_CUDA_TRY(cudaMemsetAsync(parent, 0xff, sizeof(int) * nn, st));
-        RZK_CUDA_TRY(cudaMemsetAsync(s->d_ctrav, 0, bytes, st));
         const unsigned grid = (unsigned)((nn + 255) / 256);
         closest_leaves_kernel<<<grid, 256, 0, st>>>(n, s->d_trav, s->d_tri_isect, inf, s->d_ctrav, parent);
         closest_refit_kernel<<<grid, 256, 0, st>>>(n, s->d_trav, s->d_ctrav, parent, count, cost);
