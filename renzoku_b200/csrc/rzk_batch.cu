@@ -200,6 +200,7 @@ struct BatchPlan {
     size_t sorted_vpls = 0;
     int max_order_total = 0;
     int vis_grid = 0;              // resident grid of the two-pass tracing kernel
+    int launched = 0;              // kernels of the last launch
     size_t partial_floats = 0;
     float *bound = nullptr;        // partial buffer the tables point into
     void *order_bound = nullptr;   // ordering buffer the ordered jobs point into
@@ -288,8 +289,10 @@ rzk_status batch_plan_create(const rzk_gather_job *jobs, int n_jobs, int chunk_l
     return RZK_OK;
 }
 
-// Two passes for a table within the ballots' budget (64 M words, 256 MB), the items as in
-// rzk_gather: about twenty per resident warp.
+// Two passes for a table within the ballots' budget (64 M words, 256 MB) as a whole, the tracing
+// items as long as in rzk_gather (about twenty per resident warp).  rzk_gather itself goes by the
+// one-pass items each resident warp gets; here the tables' jobs share their launches, and the line
+// has only been drawn by memory: ten jobs of up to 192 x 192 x 3,000 take 24.0 ms.
 constexpr long long kBatchMaskWords = 64ll << 20;
 size_t batch_plan_mask_words(const BatchPlan *p) {
     long long most = 0;
@@ -328,11 +331,7 @@ size_t batch_plan_order_bytes(const BatchPlan *p) {
     return up256(sizeof(rzk_vpl) * p->sorted_vpls) + order_scratch_bytes(p->max_order_total);
 }
 int batch_plan_tables(const BatchPlan *p) { return (int)p->tables.size(); }
-int batch_plan_launches(const BatchPlan *p) {
-    int n = 0;
-    for (const OrderTable &o : p->orders) n += 2 + order_launches(o);
-    return n;   // one more per table launched in two passes
-}
+int batch_plan_launches(const BatchPlan *p) { return p->launched; }
 
 rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *work, uint32_t *masks, int variant, int grid,
                              cudaStream_t st) {
@@ -356,11 +355,14 @@ rzk_status batch_plan_launch(BatchPlan *p, float *partial, void *order, int *wor
     RZK_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int) * p->tables.size(), st));
     if (masks && variant == 0 && p->vis_grid == 0) p->vis_grid = vis_grid();
     const int vgrid = masks && variant == 0 ? p->vis_grid : 0;
+    p->launched = 0;
     for (size_t k = 0; k < p->tables.size(); ++k) {
         JobTable &t = p->tables[k];
         int *w = work + k;
+        p->launched += 2 + order_launches(p->orders[k]);
         if (p->orders[k].total > 0) RZK_TRY(order_vpls(p->orders[k], scratch, sorted + p->order_base[k], st));
         if (vgrid > 0 && plan_vis(t, vgrid)) {
+            p->launched++;
             batch_vis_kernel<4, 16, 7><<<vgrid, 128, 0, st>>>(t, w, masks);
             RZK_CUDA_TRY(cudaGetLastError());
             batch_shade_kernel<<<(unsigned)((32ll * t.n_items + kShadeBlock - 1) / kShadeBlock), kShadeBlock, 0, st>>>(

@@ -949,6 +949,7 @@ static rzk_status order_gather_vpls(rzk_context *ctx, const float *box, const rz
     OrderTable t;
     order_table_init(t);
     order_table_add(t, vpls, n_vpl, box);
+    ctx->gather_kernels += order_launches(t);
     rzk_vpl *out = (rzk_vpl *)ctx->d_order;
     RZK_TRY(order_vpls(t, (char *)ctx->d_order + vb, out, st));
     *sorted = out;
@@ -996,21 +997,6 @@ static void resolve_chunks(int n_vpl, int &n_chunks, int &chunk_len) {
     chunk_len = n_vpl > 0 ? (n_vpl + n_chunks - 1) / n_chunks : 0;
     chunk_len = (chunk_len + 127) / 128 * 128;
     if (chunk_len > 0) n_chunks = (n_vpl + chunk_len - 1) / chunk_len;
-}
-
-int gather_launches(int n_recv, int n_vpl, int n_chunks) {
-    if (n_recv <= 0) return 0;
-    int chunk_len = 0;
-    resolve_chunks(n_vpl, n_chunks, chunk_len);
-    int k = 3;   // tracing, summing, chunk reduction (one less in one pass)
-    if (n_chunks > 1) {
-        OrderTable t;
-        order_table_init(t);
-        const float box[6] = {0, 0, 0, 1, 1, 1};
-        order_table_add(t, nullptr, n_vpl, box);
-        k += order_launches(t);
-    }
-    return k;
 }
 
 // VPLs per tracing item of a two-pass gather, or 0 where one pass does.  One pass has an item per
@@ -1065,6 +1051,7 @@ static uint32_t *mask_buffer(rzk_context *ctx, long long words, cudaStream_t st)
 rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, const rzk_receiver *recv,
                          int n_recv, int img_w, const rzk_vpl *vpls, int n_vpl, int mode, float tau,
                          float scale, float *out, int variant, int n_chunks, cudaStream_t st) {
+    ctx->gather_kernels = 0;
     if (n_recv <= 0) return RZK_OK;
     if (variant < 0 || variant >= gather_variant_count()) variant = 0;
     const GatherVariant gv = kVariants[variant];
@@ -1133,6 +1120,7 @@ rzk_status launch_gather(rzk_context *ctx, const DevScene &s, const float *box, 
     RZK_CUDA_TRY(cudaGetLastError());
     reduce_chunks_kernel<<<(3 * n_recv + 255) / 256, 256, 0, st>>>(part, n_recv, n_chunks, scale, out);
     RZK_CUDA_TRY(cudaGetLastError());
+    ctx->gather_kernels += masks ? 3 : 2;   // (tracing and summing, or both in one) and the reduction
     return RZK_OK;
 }
 

@@ -120,6 +120,7 @@ struct rzk_context {
     void *d_order = nullptr;
     size_t order_bytes = 0;
     int persistent_grid[16] = {0};
+    int gather_kernels = 0;   // kernels the last gather launched
     int vis_grid = 0;   // resident grid of the two-pass gather's tracing kernel
     // ballots of two-pass gathers: buffer k holds 2^(kMaskLog0 + k) words.  None is freed before
     // the context is, so that a captured gather stays good whatever gathers run after it.
@@ -228,8 +229,6 @@ rzk_status order_vpls(const OrderTable &t, void *scratch, rzk_vpl *out, cudaStre
 rzk_status launch_matrix(const DevScene &s, int depth, const float *box, const rzk_receiver *recv, int n_recv, const rzk_vpl *vpls,
                          int n_vpl, int mode, float tau, float *mat, uint8_t *vis, int kind,
                          cudaStream_t st);
-// rzk_gather.cu: kernels one rzk_gather_cfg call launches
-int gather_launches(int n_recv, int n_vpl, int n_chunks);
 // Chunk ring of the persistent gather on fixed scratch (rzk_gather.cu, used by
 // rzk_gather_noalloc): the per-chunk sums of at most `slots` warp tiles at a time.  Tile t writes its chunks to slot t % slots once the slot
 // has finished t / slots tiles (`round`); the warp that writes a tile's last chunk (`done`)
@@ -261,7 +260,7 @@ void batch_plan_destroy(BatchPlan *p);
 size_t batch_plan_partial_floats(const BatchPlan *p);
 size_t batch_plan_order_bytes(const BatchPlan *p);
 int batch_plan_tables(const BatchPlan *p);
-int batch_plan_launches(const BatchPlan *p);   // kernels one batch_plan_launch launches
+int batch_plan_launches(const BatchPlan *p);   // kernels the plan's last batch_plan_launch launched
 // masks: null, or batch_plan_mask_words words, with which the tables that a two-pass launch
 // suits run in two passes (as rzk_gather does; variant 0 only, the same images).
 size_t batch_plan_mask_words(const BatchPlan *p);
