@@ -617,6 +617,9 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
             s->d_ctrav = nullptr;
             s->device_bytes -= s->ctrav_bytes;
         }
+        CallScratch mem;   // first: without it the scene must not be left with a tree that is not filled
+        const size_t nn = 2 * (size_t)n - 1;
+        RZK_CUDA_TRY(mem.alloc(2 * sizeof(double) + 2 * sizeof(int) * nn, st));
         if (!s->d_ctrav) {
             RZK_CUDA_TRY(cudaMalloc((void **)&s->d_ctrav, bytes));
             s->ctrav_bytes = bytes;
@@ -630,9 +633,6 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
         inf.pad = 1e-6f * (top + radius) + 6e-6f * inf.D;
         for (int d = 0; d < 3; ++d) s->cguard[d] = c[d];
         s->cguard[3] = radius * radius;
-        CallScratch mem;
-        const size_t nn = 2 * (size_t)n - 1;
-        RZK_CUDA_TRY(mem.alloc(2 * sizeof(double) + 2 * sizeof(int) * nn, st));
         double *cost = (double *)mem.get();
         int *count = (int *)(cost + 2), *parent = count + nn;
         RZK_CUDA_TRY(cudaMemsetAsync(cost, 0, 2 * sizeof(double) + sizeof(int) * nn, st));
