@@ -16,6 +16,9 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <new>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 namespace rzk {
@@ -165,6 +168,24 @@ bool tree_ok(const char *nodes, int64_t nn, int n, int &depth) {
     return true;
 }
 
+bool perm_ok(const char *perm, int n) {
+    for (int i = 0; i < n; ++i) {
+        int32_t t;
+        std::memcpy(&t, perm + sizeof(t) * (size_t)i, sizeof(t));
+        if (t < 0 || t >= n) return false;
+    }
+    return true;
+}
+
+bool lights_ok(const char *lights, int n) {
+    for (int i = 0; i < n; ++i) {
+        DevLight l;
+        std::memcpy(&l, lights + sizeof(l) * (size_t)i, sizeof(l));
+        if (l.n_tris < 1 || l.n_tris > 2) return false;
+    }
+    return true;
+}
+
 void free_arrays(rzk_scene *s) {
     for (const Array &a : scene_arrays(s))
         if (*a.ptr) { cudaFree(*a.ptr); *a.ptr = nullptr; }
@@ -256,35 +277,51 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
         if (sizes[k] != 0 && sizes[k] != expect) return fail(RZK_ERR_INVALID);
         if (sizes[k] == 0 && expect != 0 && !is_wide && !is_trav) return fail(RZK_ERR_INVALID);
     }
-    // what the restore's own kernels and the walks index with
+    // What the restore's own kernels and the walks index with is checked while the arrays are
+    // copied (300k triangles: 3.5 ms of a 25 ms restore).
     const char *base = (const char *)h_buf;
-    for (size_t k = 0; k < arrays.size(); ++k) {
-        if (sizes[k] == 0) continue;
-        const char *p = base + offs[k];
-        int depth = 0;
-        if (arrays[k].ptr == (void **)&s->d_nodes && !tree_ok(p, h.n_nodes, h.n_tris, depth)) return fail(RZK_ERR_INVALID);
-        if (arrays[k].ptr == (void **)&s->d_trav) {
-            if (!tree_ok(p, 2 * (int64_t)h.n_tris - 1, h.n_tris, depth)) return fail(RZK_ERR_INVALID);
-            s->trav_depth = depth;   // sizes the walks' stacks
+    auto data = [&](void *ptr) -> const char * {
+        for (size_t k = 0; k < arrays.size(); ++k)
+            if (arrays[k].ptr == ptr) return sizes[k] ? base + offs[k] : nullptr;
+        return nullptr;
+    };
+    const char *h_nodes = data(&s->d_nodes), *h_trav = data(&s->d_trav), *h_perm = data(&s->d_perm),
+               *h_lights = data(&s->d_lights);
+    rzk_status checked = RZK_OK;
+    int depth = h.trav_depth;
+    auto check = [&, h]() {
+        try {
+            int unused = 0;
+            if ((h_nodes && !tree_ok(h_nodes, h.n_nodes, h.n_tris, unused)) ||
+                (h_trav && !tree_ok(h_trav, 2 * (int64_t)h.n_tris - 1, h.n_tris, depth)) ||
+                (h_perm && !perm_ok(h_perm, h.n_tris)) || (h_lights && !lights_ok(h_lights, h.n_lights)))
+                checked = RZK_ERR_INVALID;
+        } catch (const std::bad_alloc &) {
+            checked = RZK_ERR_NOMEM;
         }
-        if (arrays[k].ptr == (void **)&s->d_perm)
-            for (int i = 0; i < h.n_tris; ++i) {
-                int32_t t;
-                std::memcpy(&t, p + sizeof(t) * (size_t)i, sizeof(t));
-                if (t < 0 || t >= h.n_tris) return fail(RZK_ERR_INVALID);
-            }
-        if (arrays[k].ptr == (void **)&s->d_lights)
-            for (int i = 0; i < h.n_lights; ++i) {
-                DevLight l;
-                std::memcpy(&l, p + sizeof(l) * (size_t)i, sizeof(l));
-                if (l.n_tris < 1 || l.n_tris > 2) return fail(RZK_ERR_INVALID);
-            }
+    };
+    struct Checker {
+        std::thread t;
+        ~Checker() { join(); }
+        void join() {
+            if (t.joinable()) t.join();
+        }
+    } checker;
+    try {
+        checker.t = std::thread(check);
+    } catch (const std::system_error &) {
+        check();
     }
+    // a blob that is not whole is refused whatever became of the copies
+    auto failed = [&](rzk_status e) {
+        checker.join();
+        return fail(checked != RZK_OK ? checked : e);
+    };
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) {
         set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
-        return fail(RZK_ERR_CUDA);
+        return failed(RZK_ERR_CUDA);
     }
     for (size_t k = 0; k < arrays.size(); ++k) {
         if (sizes[k] == 0) continue;
@@ -292,21 +329,24 @@ rzk_status rzk_scene_deserialize(rzk_context *ctx, const void *h_buf, size_t siz
         e = cudaMalloc(arrays[k].ptr, std::max<size_t>((size_t)sizes[k], 16));
         if (e != cudaSuccess) {
             set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
-            return fail(RZK_ERR_NOMEM);
+            return failed(RZK_ERR_NOMEM);
         }
         s->device_bytes += (size_t)sizes[k];
         e = cudaMemcpyAsync(*arrays[k].ptr, base + offs[k], (size_t)sizes[k], cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) {
             set_last_cuda_error(e, "scene restore", __FILE__, __LINE__);
-            return fail(RZK_ERR_CUDA);
+            return failed(RZK_ERR_CUDA);
         }
     }
     if (!s->d_mats) {   // n_mats == 0: rzk_scene_create holds a 16-byte stand-in
         e = cudaMalloc((void **)&s->d_mats, 16);
-        if (e != cudaSuccess) return fail(RZK_ERR_NOMEM);
+        if (e != cudaSuccess) return failed(RZK_ERR_NOMEM);
     }
     for (void **p : {(void **)&s->d_v, (void **)&s->d_tp, (void **)&s->d_tri_surf})
-        if (!*p && (e = cudaMalloc(p, 16)) != cudaSuccess) return fail(RZK_ERR_NOMEM);
+        if (!*p && (e = cudaMalloc(p, 16)) != cudaSuccess) return failed(RZK_ERR_NOMEM);
+    checker.join();
+    if (checked != RZK_OK) return fail(checked);
+    s->trav_depth = depth;   // sizes the walks' stacks
     rzk_status r = build_closest_tree(s, st);
     if (r == RZK_OK) r = build_wide_tree(s, st);
     if (r != RZK_OK) return fail(r);
