@@ -40,18 +40,18 @@ TAU_PAIRS = 65536
 # DRAM bytes (read + write) of one full gather launch of this workload, from the one-pass
 # capture `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
 # -k regex:gather_persistent -s 3 -c 1 python bench.py --steps 1 --warmup 3 --skip-cpu
-# --serve-duration 0` (37.60 MB read, 65.28 MB written; the writes are the per-chunk partial
+# --serve-duration 0` (37.52 MB read, 65.42 MB written; the writes are the per-chunk partial
 # sums), recorded in profiles/.
-TRAFFIC_BYTES_PER_LAUNCH = (37.60 + 65.28) * 1e6
+TRAFFIC_BYTES_PER_LAUNCH = (37.52 + 65.42) * 1e6
 # Warp instructions of one full gather launch of this workload (smsp__inst_executed.sum from
 # the same one-pass capture, recorded in profiles/): the gather is instruction-issue bound
 # (HBM idle, its ~34 MB working set in L2), so the roofline compares the issue rate it
 # reaches with the SMs' peak of one warp instruction per scheduler per cycle.
-INST_PER_LAUNCH = 35667965828
+INST_PER_LAUNCH = 35864286964
 # The same for the secondary workloads' dominant kernels (one full launch each, same capture
 # recipe; see profiles/): LightSlice's and MRCS's tracing passes and the guided path kernel.
-LS_VIS_INST = 2803614703
-MRCS_VIS_INST = 618058667
+LS_VIS_INST = 2812700255
+MRCS_VIS_INST = 618861952
 GUIDED_INST = 164980217897
 
 

@@ -75,7 +75,8 @@ rzk_status rzk_scene_info(const rzk_scene *scene, int *n_tris, int *n_nodes, int
 rzk_status rzk_scene_bounding_box(const rzk_scene *scene, float *box);
 
 /* Re-runs the LBVH build on the resident triangles (timing / rebuild after edits).
- * Same result as rzk_scene_create. Synchronises `stream`. */
+ * Same result as rzk_scene_create; queries launched before on other streams keep their
+ * answers.  Synchronises `stream`. */
 rzk_status rzk_scene_rebuild(rzk_scene *scene, void *stream);
 
 /* Copies the BVH to host buffers in the reference's layout (BvhNode,

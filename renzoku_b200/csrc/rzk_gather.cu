@@ -1143,7 +1143,13 @@ rzk_status launch_matrix(const DevScene &s, int depth, const float *box, const r
     // Packets pay where the scene is large and 32 neighbours of the VPLs' order are near one another
     // (us, B200, one thread a pair and packets, the ordering included): 260 x 10,007 on 300k
     // triangles 975 and 650, 75k 907 and 769, 15k 790 and 924; 260 x 4,097 on 300k 425 and 466;
-    // 96 x 4,000 194 and 403.  They need scratch, so a captured call goes without.
+    // 96 x 4,000 194 and 403.  Either side of the lines in another run (66k / 150k / 300k triangles):
+    // 60 x 100,000 2,312 and 1,152 / 2,493 and 1,147 / 2,417 and 1,065; 100 x 21,000 793 and 729 /
+    // 905 and 750 / 856 and 684; 256 x 8,192 801 and 919 / 889 and 986 / 882 and 840; 350 x 6,000
+    // (below the VPLs' line) 801 and 1,006 / 900 and 998 / 876 and 841; 130 x 8,192 (below the
+    // pairs') 430 and 597 / 474 and 639 / 468 and 646.  So packets gain with the VPLs, and at the
+    // corner of both lines they are up to 15 % behind.  They need scratch, so a captured call goes
+    // without.
     constexpr size_t kPacketPairs = 2u << 20;
     constexpr int kPacketVpls = 8192, kPacketTris = 64 << 10;
     cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;

@@ -27,7 +27,9 @@
 // others run joins the lane's very next group.  A host function after a
 // group's last kernel marks its requests done.  With batching off the worker issues one
 // request at a time in arrival order, with its own launches, on one stream (the plain
-// per-request baseline).  Scratch comes from the stream-ordered allocator, whose pool keeps
+// per-request baseline; the ballots of its gathers in two passes, at most 512 MB that its context
+// keeps, are not in the admission's account, and without room for them a gather runs in one).
+// Scratch comes from the stream-ordered allocator, whose pool keeps
 // freed blocks, so an iteration neither blocks on an allocation nor synchronises the device.
 #include "rzk_internal.cuh"
 
