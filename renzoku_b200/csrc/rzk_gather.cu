@@ -1040,11 +1040,16 @@ static uint32_t *mask_buffer(rzk_context *ctx, long long words, cudaStream_t st)
     for (int k = first; k <= rzk_context::kMaskLogMax - rzk_context::kMaskLog0; ++k)
         if (ctx->d_masks[k]) return ctx->d_masks[k];
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-        cudaMalloc((void **)&ctx->d_masks[first], sizeof(uint32_t) << (rzk_context::kMaskLog0 + first)) != cudaSuccess) {
-        (void)cudaGetLastError();
-        ctx->d_masks[first] = nullptr;
+    cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        // relaxed: another thread's capture must not be broken by this allocation
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        e = cudaMalloc((void **)&ctx->d_masks[first], sizeof(uint32_t) << (rzk_context::kMaskLog0 + first));
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) ctx->d_masks[first] = nullptr;
     }
+    if (e != cudaSuccess) (void)cudaGetLastError();
     return ctx->d_masks[first];
 }
 

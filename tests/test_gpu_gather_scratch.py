@@ -1,7 +1,8 @@
 """The gather's scratch under stream capture: a two-pass gather (variant 0) is captured wherever the
-context's buffers hold a one-pass gather of its size, and captured gathers stay good when later
-gathers need more ballots."""
+context's buffers hold a one-pass gather of its size, captured gathers stay good when later
+gathers need more ballots, and ballots allocated beside another thread's capture do not break it."""
 import dataclasses
+import threading
 
 import pytest
 
@@ -61,4 +62,33 @@ def test_captured_gathers_outlive_larger_ballots(case, variant):
         torch.cuda.synchronize()
         assert torch.equal(out, want) and bool((fill == 7).all())
         del fill
+    ctx.check()
+
+
+def test_ballots_beside_another_capture(case):
+    import torch
+    ctx, ev, recv, vpls = case
+    want = ev.gather(recv, 4096, vpls, 1000, image_width=64, variant=3)   # its buffers, without ballots
+    other, out = torch.cuda.Stream(), torch.zeros((4096, 3), dtype=torch.float32, device="cuda")
+    x = torch.zeros(1000, device="cuda")
+    errors = []
+
+    def gather():
+        try:
+            ev.gather(recv, 4096, vpls, 1000, image_width=64, out=out, stream=other)
+        except Exception as e:
+            errors.append(repr(e))
+
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        x += 1
+        t = threading.Thread(target=gather)
+        t.start()
+        t.join()
+        x += 1
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert not errors and torch.equal(out, want) and bool((x == 2).all())
     ctx.check()
