@@ -36,6 +36,7 @@ cudaError_t CallScratch::alloc(size_t bytes, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kPoolDevices) return cudaErrorInvalidDevice;
     DevicePool &d = g_pools[dev];
+    RelaxedCapture relaxed;
     cudaMemPool_t pool;
     {
         std::lock_guard<std::mutex> g(d.lock);

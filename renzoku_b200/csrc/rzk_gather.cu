@@ -1042,11 +1042,8 @@ static uint32_t *mask_buffer(rzk_context *ctx, long long words, cudaStream_t st)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(st, &cap);
     if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-        // relaxed: another thread's capture must not be broken by this allocation
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        RelaxedCapture relaxed;
         e = cudaMalloc((void **)&ctx->d_masks[first], sizeof(uint32_t) << (rzk_context::kMaskLog0 + first));
-        (void)cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) ctx->d_masks[first] = nullptr;
     }
     if (e != cudaSuccess) (void)cudaGetLastError();

@@ -22,6 +22,20 @@ namespace rzk {
 
 void set_last_cuda_error(cudaError_t e, const char *what, const char *file, int line);
 
+// While it lives, allocations of this thread do not break a stream capture that another thread has
+// in progress (they are "potentially unsafe" calls, which a capture in global mode, the default,
+// is invalidated by).
+class RelaxedCapture {
+public:
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode_); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // Device scratch of one call, ordered on the call's stream: taken from a memory pool that the
 // library keeps per device and given back to it, on the same stream, when the object dies.
 // A cudaMalloc and cudaFree pair costs 100-400 us each and waits for the whole device (VPL
@@ -40,7 +54,9 @@ public:
     CallScratch &operator=(const CallScratch &) = delete;
     ~CallScratch() { release(); }
     void release() {   // after the last kernel that uses the memory has been launched
-        if (p_) cudaFreeAsync(p_, st_);
+        if (!p_) return;
+        RelaxedCapture relaxed;
+        cudaFreeAsync(p_, st_);
         p_ = nullptr;
     }
     cudaError_t alloc(size_t bytes, cudaStream_t st);   // once per object, on the current device
