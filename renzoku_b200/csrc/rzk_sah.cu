@@ -590,13 +590,23 @@ __global__ void wide8_fill_kernel(int nn, const float4 *tree, const int *flag, c
     }
 }
 
+static rzk_status drop_closest_tree(rzk_scene *s) {
+    if (s->d_ctrav) {
+        cudaFree(s->d_ctrav);
+        s->d_ctrav = nullptr;
+        s->device_bytes -= s->ctrav_bytes;
+        s->ctrav_bytes = 0;
+    }
+    return RZK_OK;
+}
+
 // Makes the closest-hit tree from the any-hit tree (on a fresh build and on a restored scene);
 // leaves the scene without one where closest hits are better off in the reference's order: no
 // any-hit tree, few triangles (36: 740 us for 4 M rays in the reference's order, 880 in this
 // one; 3,012: 1,420 and 1,060), a reference tree near the traversal stack's depth (whose dropped
-// pushes are part of its answer), coordinates the bound cannot handle, or boxes inflated so far
-// (large slanted triangles, or a scene in large units) that a ray would visit kMaxInflation times
-// as many nodes (the rooms here: 1.00 to 1.15 times).
+// pushes are part of its answer), coordinates the bound cannot handle, no memory for it, or boxes
+// inflated so far (large slanted triangles, or a scene in large units) that a ray would visit
+// kMaxInflation times as many nodes (the rooms here: 1.00 to 1.15 times).
 rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
     constexpr double kMaxInflation = 2.5;
     constexpr int kMinTris = 128;
@@ -617,11 +627,18 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
             s->d_ctrav = nullptr;
             s->device_bytes -= s->ctrav_bytes;
         }
-        CallScratch mem;   // first: without it the scene must not be left with a tree that is not filled
         const size_t nn = 2 * (size_t)n - 1;
-        RZK_CUDA_TRY(mem.alloc(2 * sizeof(double) + 2 * sizeof(int) * nn, st));
-        if (!s->d_ctrav) {
-            RZK_CUDA_TRY(cudaMalloc((void **)&s->d_ctrav, bytes));
+        CallScratch mem;   // first: without it the scene must not be left with a tree that is not filled
+        cudaError_t e = mem.alloc(2 * sizeof(double) + 2 * sizeof(int) * nn, st);
+        const bool make = e == cudaSuccess && !s->d_ctrav;
+        if (make) e = cudaMalloc((void **)&s->d_ctrav, bytes);
+        if (e == cudaErrorMemoryAllocation) {   // a scene that fits without the tree does without it
+            (void)cudaGetLastError();
+            if (make) s->d_ctrav = nullptr;
+            return drop_closest_tree(s);
+        }
+        RZK_CUDA_TRY(e);
+        if (make) {
             s->ctrav_bytes = bytes;
             s->device_bytes += bytes;
             // slot 0; the kernels write every node (not cleared on a rebuild: queries may be reading)
@@ -647,13 +664,7 @@ rzk_status build_closest_tree(rzk_scene *s, cudaStream_t st) {
         RZK_CUDA_TRY(cudaStreamSynchronize(st));
         if (h[1] <= kMaxInflation * h[0]) return RZK_OK;
     }
-    if (s->d_ctrav) {
-        cudaFree(s->d_ctrav);
-        s->d_ctrav = nullptr;
-        s->device_bytes -= s->ctrav_bytes;
-        s->ctrav_bytes = 0;
-    }
-    return RZK_OK;
+    return drop_closest_tree(s);
 }
 
 // Makes the packet gathers' 8-wide tree from the any-hit tree (from the reference's where there is
