@@ -167,7 +167,7 @@ void launch_group(rzk_server *s, Group *g) {
         } else if (!s->prm.batching) {
             q->status = rzk_gather_cfg(s->ctx, r.scene, q->d_recv, r.camera.width * r.camera.height, r.camera.width,
                                        r.d_vpls, r.n_vpl, r.clamp_mode, r.tau, r.scale, r.d_rgb, 0, 0, st);
-            g->launches += s->ctx->gather_kernels;
+            if (q->status == RZK_OK) g->launches += s->ctx->gather_kernels;
         } else {
             gathers.push_back(q);
         }
